@@ -25,9 +25,11 @@
 // and `partition`, as every pass of the windowed form skips them.  Scatter
 // with repeated destinations keeps one of the colliding values (unspecified
 // which), as the reference's racing stores do.
+#include <algorithm>
 #include <mutex>
 
 #include "common.cuh"
+#include "gather_scatter.h"
 #include "tune.h"
 
 namespace edpp {
@@ -694,24 +696,21 @@ int part_run(const int32_t *in, int32_t *out, int64_t n, const int32_t *loc, int
 
 // ==== shared-memory windows ("tiled" form) ===========================================
 //
-// The random side of the access moves from L2 into shared memory.  Pairs are
-// partitioned twice by their key's window -- coarse windows of 128 fine
-// windows, then fine windows of W = 2^14 (or 2^15) elements -- and one block
-// per fine window applies its pairs inside a shared-memory copy of that
-// window, so every global access is a streaming one:
+// The random side of the scatter moves from L2 into shared memory (the tiled
+// gather is in gather_tiled.cu).  Pairs are partitioned twice by their
+// destination's window -- coarse windows of 128 fine windows, then fine
+// windows of W = 2^14 (or 2^15) elements -- and one block per fine window
+// applies its pairs inside a shared-memory copy of that window, so every
+// global access is a streaming one:
 //
-//   scatter: count fine windows of loc -> scan -> partition {loc, in[i]} by
-//            coarse window -> refine by fine window -> apply: per window,
-//            out-window[loc - base] = value in shared memory, then store the
-//            written elements of the window (bitmap), coalesced
-//   gather:  count -> scan -> partition {loc, i} -> refine -> fetch: per
-//            window of in[], load it once and emit {i, in[loc]} grouped by
-//            the coarse window of i -> refine by fine window of i -> apply
+//   count fine windows of loc -> scan -> partition {loc, in[i]} by coarse
+//   window -> refine by fine window -> apply: per window,
+//   out-window[loc - base] = value in shared memory, then store the written
+//   elements of the window (bitmap), coalesced
 //
-// Streaming traffic per element: scatter ~48 B, gather ~80 B; no random
-// global access.  Within a window, pairs arrive in no particular order (the
-// per-window cursors are claimed atomically): every destination of a gather
-// is written once; a scatter with repeated destinations keeps one of the
+// Streaming traffic: ~44 B per element; no random global access.  Within a
+// window, pairs arrive in no particular order (the per-window cursors are
+// claimed atomically): a scatter with repeated destinations keeps one of the
 // colliding values, as the other forms do.
 constexpr int kWinThreads = 512;
 constexpr int kFineMinLog = 14;
@@ -766,12 +765,10 @@ __global__ void __launch_bounds__(kWinThreads)
 }
 
 // start[f] = sum of cnt[0..f), start[F] = total; fill = start; cfill[c] =
-// start[c * 128]; gather also gets fill2[f] = f * W and cfill2[c] = c * 128 W.
+// start[c * 128].
 __global__ void __launch_bounds__(1024)
-    win_scan_kernel(const uint32_t *__restrict__ cnt, int F, int C, int fine_log, int coarse_log,
-                    uint32_t *__restrict__ start, uint32_t *__restrict__ fill,
-                    uint32_t *__restrict__ cfill, uint32_t *__restrict__ fill2,
-                    uint32_t *__restrict__ cfill2) {
+    win_scan_kernel(const uint32_t *__restrict__ cnt, int F, uint32_t *__restrict__ start,
+                    uint32_t *__restrict__ fill, uint32_t *__restrict__ cfill) {
   __shared__ uint32_t wsum[32];
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
   const int per = (F + 1023) / 1024;  // <= kMaxFine / 1024
@@ -816,20 +813,14 @@ __global__ void __launch_bounds__(1024)
       run += v[k];
     }
   }
-  if (fill2) {
-    for (int i = t; i < F; i += 1024) fill2[i] = static_cast<uint32_t>(i) << fine_log;
-    for (int c = t; c < C; c += 1024) cfill2[c] = static_cast<uint32_t>(c) << coarse_log;
-  }
 }
 
 // Append every pair of one tile to fine window (pair.x >> fine_log) at that
 // window's cursor, as two arrays: the offset of pair.x inside its window
 // (16 bits: windows are at most 2^15 elements) and pair.y.  Six bytes per
 // pair instead of eight, on the write here and on the read of every later
-// stage.  The tiles ("slots") are either the flat range [0, *total)
-// cut into kTile pairs, or, with region_log > 0, each region
-// [r << region_log, region_end[r]) cut the same way (slots past a region's
-// end are empty).  Either way the pairs are ordered by coarse window
+// stage.  The tiles ("slots") are the flat range [0, *total)
+// cut into kTile pairs.  The pairs are ordered by coarse window
 // (pair.x >> coarse_log), so a slot's fine windows lie in the coarse windows
 // of its first and last pair.  Persistent blocks take slots blockIdx,
 // +gridDim, ...; the slot after next is copied into shared memory by TMA
@@ -841,18 +832,10 @@ __global__ void __launch_bounds__(1024)
 constexpr int kRefineSpan = 512;
 constexpr int kRefineBlocksPerSm = 3;
 
-__device__ __forceinline__ void refine_range(int64_t slot, const uint32_t *total_p,
-                                             const uint32_t *region_end, int region_log,
-                                             int64_t &lo, int64_t &hi) {
-  if (region_log > 0) {
-    const int shift = region_log - 12;  // kTile = 4096 = 2^12
-    const int64_t r = slot >> shift;
-    lo = (r << region_log) + ((slot & ((int64_t{1} << shift) - 1)) << 12);
-    hi = min64(lo + kTile, static_cast<int64_t>(region_end[r]));
-  } else {
-    lo = slot * kTile;
-    hi = min64(lo + kTile, static_cast<int64_t>(*total_p));
-  }
+__device__ __forceinline__ void refine_range(int64_t slot, const uint32_t *total_p, int64_t &lo,
+                                             int64_t &hi) {
+  lo = slot * kTile;
+  hi = min64(lo + kTile, static_cast<int64_t>(*total_p));
 }
 
 // Thread 0: start the bulk copy of the even part of [lo, hi) into buf.
@@ -867,8 +850,7 @@ __device__ __forceinline__ void refine_issue(const int2 *src, int64_t lo, int64_
 
 __global__ void __launch_bounds__(kThreads, kRefineBlocksPerSm)
     win_refine_kernel(const int2 *__restrict__ src, const uint32_t *__restrict__ total_p,
-                      const uint32_t *__restrict__ region_end, int region_log, int fine_log,
-                      int coarse_log, int64_t slots, uint32_t *__restrict__ fill,
+                      int fine_log, int coarse_log, int64_t slots, uint32_t *__restrict__ fill,
                       uint16_t *__restrict__ dst_off, int32_t *__restrict__ dst_val,
                       uint64_t timeout_ns, unsigned *fault) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -892,7 +874,7 @@ __global__ void __launch_bounds__(kThreads, kRefineBlocksPerSm)
       const int64_t sk = blockIdx.x + k * G;
       if (sk < slots) {
         int64_t lo, hi;
-        refine_range(sk, total_p, region_end, region_log, lo, hi);
+        refine_range(sk, total_p, lo, hi);
         refine_issue(src, lo, hi, bufs + k * kTile, &bar[k]);
       }
     }
@@ -904,7 +886,7 @@ __global__ void __launch_bounds__(kThreads, kRefineBlocksPerSm)
   bool failed = false;
   for (; slot < slots; slot += G, b ^= 1) {
     int64_t lo, hi;
-    refine_range(slot, total_p, region_end, region_log, lo, hi);
+    refine_range(slot, total_p, lo, hi);
     int2 *buf = bufs + b * kTile;
     if (lo < hi) {  // block-uniform
       const uint32_t cnt = static_cast<uint32_t>(hi - lo);
@@ -984,7 +966,7 @@ __global__ void __launch_bounds__(kThreads, kRefineBlocksPerSm)
       const int64_t sn = slot + 2 * G;
       if (sn < slots) {
         int64_t lo2, hi2;
-        refine_range(sn, total_p, region_end, region_log, lo2, hi2);
+        refine_range(sn, total_p, lo2, hi2);
         refine_issue(src, lo2, hi2, buf, &bar[b]);
       }
     }
@@ -994,41 +976,34 @@ __global__ void __launch_bounds__(kThreads, kRefineBlocksPerSm)
     const int64_t sn = slot + G;
     if (sn < slots) {
       int64_t lo2, hi2;
-      refine_range(sn, total_p, region_end, region_log, lo2, hi2);
+      refine_range(sn, total_p, lo2, hi2);
       if (lo2 < hi2 && ((static_cast<uint32_t>(hi2 - lo2) & ~1u) != 0u))
         mbar_wait_bounded(&bar[b ^ 1], (phase >> (b ^ 1)) & 1u, timeout_ns, fault);
     }
   }
 }
 
-// One block per fine window f: pairs [start[f], start[f+1]) (or, without
-// start, [f << fine_log, fill_end[f])) are {offset in the window, value}
-// (two arrays, as the refine writes them); they are applied in shared memory and the written elements of
-// the window are stored (a bitmap marks them; untouched elements keep their
-// old value in `out`).  unique: no index repeats (a gather's return trip),
-// so a window with as many pairs as elements is written whole and needs no
-// bitmap.
+// One block per fine window f: pairs [start[f], start[f+1]) are {offset in the
+// window, value} (two arrays, as the refine writes them); they are applied in
+// shared memory and the written elements of the window are stored (a bitmap
+// marks them; untouched elements keep their old value in `out`).
 __global__ void __launch_bounds__(kWinThreads)
     win_apply_kernel(const uint16_t *__restrict__ poff, const int32_t *__restrict__ pval,
-                     const uint32_t *__restrict__ start, const uint32_t *__restrict__ fill_end,
-                     int fine_log, int64_t n, int32_t *__restrict__ out, bool vec_out,
-                     bool unique) {
+                     const uint32_t *__restrict__ start, int fine_log, int64_t n,
+                     int32_t *__restrict__ out, bool vec_out) {
   extern __shared__ __align__(16) int32_t win[];
   const int W = 1 << fine_log;
   uint32_t *bits = reinterpret_cast<uint32_t *>(win + W);
   const int f = blockIdx.x;
   const int64_t base = static_cast<int64_t>(f) << fine_log;
   const int len = static_cast<int>(min64(W, n - base));
-  const int64_t lo = start ? start[f] : base;
-  const int64_t hi = start ? start[f + 1] : fill_end[f];
-  const bool whole = unique && hi - lo == len;  // block-uniform
+  const int64_t lo = start[f], hi = start[f + 1];
   const int t = threadIdx.x;
-  if (!whole)
-    for (int i = t; i < (W >> 5); i += kWinThreads) bits[i] = 0u;
+  for (int i = t; i < (W >> 5); i += kWinThreads) bits[i] = 0u;
   __syncthreads();
   auto put = [&](uint32_t rel, int32_t v) {
     win[rel] = v;
-    if (!whole) atomicOr(&bits[rel >> 5], 1u << (rel & 31));
+    atomicOr(&bits[rel >> 5], 1u << (rel & 31));
   };
   // pairs: a scalar head up to a multiple of 8, then groups of 8 (one 16-byte
   // load of offsets, two of values; both arrays are 16-byte aligned), then a
@@ -1064,7 +1039,7 @@ __global__ void __launch_bounds__(kWinThreads)
   for (int64_t q = head + 8 * ng + t; q < hi; q += kWinThreads) put(poff[q], pval[q]);
   __syncthreads();
   for (int e0 = 4 * t; e0 < len; e0 += 4 * kWinThreads) {
-    const uint32_t nib = whole ? 0xFu : (bits[e0 >> 5] >> (e0 & 31)) & 0xFu;
+    const uint32_t nib = (bits[e0 >> 5] >> (e0 & 31)) & 0xFu;
     if (nib == 0xFu && vec_out && e0 + 3 < len) {
       __stcs(reinterpret_cast<int4 *>(out + base + e0), *reinterpret_cast<const int4 *>(win + e0));
     } else {
@@ -1075,104 +1050,10 @@ __global__ void __launch_bounds__(kWinThreads)
   }
 }
 
-// Gather fetch: one block per fine window f of in[]; the window is loaded
-// once into shared memory, and each pair {loc, i} of the window (the offset
-// of loc in the window and i, in two arrays) becomes
-// {i, in[loc]}, appended to the coarse window of i (cursors cfill2).  The
-// window's pairs go in sub-tiles of kTile; each sub-tile's pairs are loaded
-// into registers while the previous one is grouped (the first while the
-// window lands).
-constexpr int kFetchThreads = 512;
-constexpr int kFetchPer = kTile / kFetchThreads;  // 8 pairs per thread per sub-tile
-
-__global__ void __launch_bounds__(kFetchThreads)
-    win_fetch_kernel(const uint16_t *__restrict__ poff, const int32_t *__restrict__ pidx,
-                     const uint32_t *__restrict__ start,
-                     const int32_t *__restrict__ in, int64_t n, int fine_log, int coarse_log,
-                     int C, uint32_t *__restrict__ cfill2, int2 *__restrict__ dst, bool vec_in,
-                     uint64_t timeout_ns, unsigned *fault) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  const int W = 1 << fine_log;
-  int32_t *win = reinterpret_cast<int32_t *>(smem);
-  int2 *stage = reinterpret_cast<int2 *>(win + W);
-  uint32_t *scnt = reinterpret_cast<uint32_t *>(stage + kTile);
-  uint32_t *soff = scnt + C;
-  uint32_t *sgb = soff + C;
-  __shared__ uint32_t s_total;
-  __shared__ alignas(8) uint64_t bar;
-  const int f = blockIdx.x, t = threadIdx.x;
-  const int64_t base = static_cast<int64_t>(f) << fine_log;
-  const int len = static_cast<int>(min64(W, n - base));
-  const int64_t lo = start[f], hi = start[f + 1];
-  if (lo >= hi) return;  // block-uniform
-  uint32_t nxt_off[kFetchPer];
-  int32_t nxt_i[kFetchPer];
-  auto load = [&](int64_t c0) {
-#pragma unroll
-    for (int e = 0; e < kFetchPer; ++e) {
-      const int64_t j = c0 + static_cast<int64_t>(e) * kFetchThreads + t;
-      nxt_off[e] = j < hi ? __ldcs(poff + j) : 0u;
-      nxt_i[e] = j < hi ? __ldcs(pidx + j) : 0;
-    }
-  };
-  // the window by one bulk copy (16-byte multiple), the rest by plain loads
-  const uint32_t bulk = vec_in ? (static_cast<uint32_t>(len) * 4u) & ~15u : 0u;
-  if (t == 0 && bulk) {
-    mbar_init(&bar, 1);
-    fence_mbar_init();
-    mbar_arrive_expect_tx(&bar, bulk);
-    tma_load_1d(win, in + base, bulk, &bar);
-  }
-  load(lo);
-  for (int e = static_cast<int>(bulk / 4) + t; e < len; e += kFetchThreads) win[e] = in[base + e];
-  for (int i = t; i < C; i += kFetchThreads) scnt[i] = 0;
-  if (t == 0) s_total = 0;
-  __syncthreads();  // barrier initialised before anyone waits on it
-  if (bulk && __syncthreads_or(!mbar_wait_bounded(&bar, 0, timeout_ns, fault))) return;
-  for (int64_t c0 = lo; c0 < hi; c0 += kTile) {
-    uint32_t ao[kFetchPer];
-    int32_t ai[kFetchPer];
-#pragma unroll
-    for (int e = 0; e < kFetchPer; ++e) {
-      ao[e] = nxt_off[e];
-      ai[e] = nxt_i[e];
-    }
-    if (c0 + kTile < hi) load(c0 + kTile);
-    int2 pr[kFetchPer];
-    int w[kFetchPer], rank[kFetchPer];
-#pragma unroll
-    for (int e = 0; e < kFetchPer; ++e) {
-      const bool valid = c0 + static_cast<int64_t>(e) * kFetchThreads + t < hi;
-      pr[e] = make_int2(ai[e], valid ? win[ao[e]] : 0);  // {i, value}
-      w[e] = valid ? (ai[e] >> coarse_log) : -1;
-      rank[e] = valid ? static_cast<int>(atomicAdd(&scnt[w[e]], 1u)) : -1;
-    }
-    __syncthreads();  // A
-    uint32_t g[1], o[1];
-    claim_runs<1, kFetchThreads>(scnt, soff, C, cfill2, &s_total, g, o);
-    __syncthreads();  // B
-    const uint32_t total = s_total;
-#pragma unroll
-    for (int e = 0; e < kFetchPer; ++e)
-      if (w[e] >= 0) stage[soff[w[e]] + rank[e]] = pr[e];
-    publish_run_bases<1, kFetchThreads>(sgb, C, g, o);
-    __syncthreads();  // C
-    if (t == 0) s_total = 0;
-    for (uint32_t q = t; q < total; q += kFetchThreads) {
-      const int2 p = stage[q];
-      dst[sgb[p.x >> coarse_log] + q] = p;
-    }
-  }
-}
-
 size_t refine_smem() {
   return 2 * static_cast<size_t>(kTile) * 8 + 3 * 4 * static_cast<size_t>(kRefineSpan);
 }
 size_t apply_smem(int fine_log) { return (size_t{4} << fine_log) + (size_t{1} << fine_log) / 8; }
-size_t fetch_smem(int fine_log, int C) {
-  return (size_t{4} << fine_log) + static_cast<size_t>(kTile) * 8 + 3 * 4 * static_cast<size_t>(C);
-}
-
 int ensure_win_attrs() {
   static std::once_flag once[64];
   static int st[64];
@@ -1187,11 +1068,7 @@ int ensure_win_attrs() {
     if (e == cudaSuccess) e = set(reinterpret_cast<const void *>(win_refine_kernel), refine_smem());
     if (e == cudaSuccess) e = set(reinterpret_cast<const void *>(win_apply_kernel), apply_smem(kFineMaxLog));
     if (e == cudaSuccess)
-      e = set(reinterpret_cast<const void *>(win_fetch_kernel), fetch_smem(kFineMaxLog, 1 << (31 - kFineMaxLog - kCoarseLogFan)));
-    if (e == cudaSuccess)
       e = set(reinterpret_cast<const void *>(part_partition_kernel<true>), part_smem(kMaxWin));
-    if (e == cudaSuccess)
-      e = set(reinterpret_cast<const void *>(part_partition_kernel<false>), part_smem(kMaxWin));
     st[dev] = e == cudaSuccess ? EDPP_OK : EDPP_ECUDA;
   });
   return st[dev];
@@ -1201,10 +1078,10 @@ int ensure_win_attrs() {
 // refine's output as 16-bit window offsets (at pairs_b) and 32-bit values
 // (at pairs_b + soa_val), both 16-byte aligned.
 struct TLayout {
-  size_t cnt, start, fill, cfill, fill2, cfill2, pairs_a, pairs_b, soa_val, bytes;
+  size_t cnt, start, fill, cfill, pairs_a, pairs_b, soa_val, bytes;
 };
 
-TLayout tlayout_of(int64_t n, const TPlan &p, bool gather) {
+TLayout tlayout_of(int64_t n, const TPlan &p) {
   TLayout L{};
   size_t o = kHdr;
   auto take = [&](size_t b) {
@@ -1216,8 +1093,6 @@ TLayout tlayout_of(int64_t n, const TPlan &p, bool gather) {
   L.start = take(4 * static_cast<size_t>(p.F + 1));
   L.fill = take(4 * static_cast<size_t>(p.F));
   L.cfill = take(4 * static_cast<size_t>(p.C));
-  L.fill2 = gather ? take(4 * static_cast<size_t>(p.F)) : 0;
-  L.cfill2 = gather ? take(4 * static_cast<size_t>(p.C)) : 0;
   L.pairs_a = take(8 * static_cast<size_t>(n));
   L.soa_val = round_up(2 * static_cast<size_t>(n), 256);
   L.pairs_b = take(L.soa_val + 4 * static_cast<size_t>(n));
@@ -1225,16 +1100,11 @@ TLayout tlayout_of(int64_t n, const TPlan &p, bool gather) {
   return L;
 }
 
-template <bool kScatter>
-int tiled_run(const int32_t *in, int32_t *out, int64_t n, const int32_t *loc, int pass, void *ws,
-              size_t ws_bytes, void *stream) {
-  if (n < 0 || pass < 0) return EDPP_EINVAL;
-  if (n == 0) return EDPP_OK;
-  if (!in || !out || !loc) return EDPP_EINVAL;
-  if (n > INT32_MAX) return EDPP_EINVAL;
-  if (!tiled_fits(n)) return part_run<kScatter>(in, out, n, loc, 0, ws, ws_bytes, stream);
+int scatter_tiled(const int32_t *in, int32_t *out, int64_t n, const int32_t *loc, void *ws,
+                  size_t ws_bytes, void *stream) {
+  if (!tiled_fits(n)) return part_run<true>(in, out, n, loc, 0, ws, ws_bytes, stream);
   const TPlan p = tplan(n);
-  const TLayout L = tlayout_of(n, p, !kScatter);
+  const TLayout L = tlayout_of(n, p);
   if (!ws || ws_bytes < L.bytes) return EDPP_ENOMEM;
   int s = ensure_win_attrs();
   if (s == EDPP_OK) s = ensure_attrs();
@@ -1245,45 +1115,36 @@ int tiled_run(const int32_t *in, int32_t *out, int64_t n, const int32_t *loc, in
   auto *start = reinterpret_cast<uint32_t *>(w + L.start);
   auto *fill = reinterpret_cast<uint32_t *>(w + L.fill);
   auto *cfill = reinterpret_cast<uint32_t *>(w + L.cfill);
-  auto *fill2 = kScatter ? nullptr : reinterpret_cast<uint32_t *>(w + L.fill2);
-  auto *cfill2 = kScatter ? nullptr : reinterpret_cast<uint32_t *>(w + L.cfill2);
   auto *pa = reinterpret_cast<int2 *>(w + L.pairs_a);
   auto *pb_off = reinterpret_cast<uint16_t *>(w + L.pairs_b);
   auto *pb_val = reinterpret_cast<int32_t *>(w + L.pairs_b + L.soa_val);
   if (cudaMemsetAsync(cnt, 0, 4 * static_cast<size_t>(p.F), st) != cudaSuccess) return EDPP_ECUDA;
   const int sms = device_sm_count();
   const bool vec_loc = aligned16(loc);
-  const bool vec_in = aligned16(in);
   const int64_t cblocks = min64(static_cast<int64_t>(sms) * 2, (n + 4 * kWinThreads - 1) / (4 * kWinThreads));
   win_count_kernel<<<static_cast<unsigned>(max64(cblocks, 1)), kWinThreads, 4 * p.F, st>>>(
       loc, n, p.fine_log, p.F, cnt, vec_loc);
-  win_scan_kernel<<<1, 1024, 0, st>>>(cnt, p.F, p.C, p.fine_log, p.coarse_log, start, fill, cfill,
-                                      fill2, cfill2);
+  win_scan_kernel<<<1, 1024, 0, st>>>(cnt, p.F, start, fill, cfill);
   const int64_t tiles = (n + kTile - 1) / kTile;
-  s = launch_partition<kScatter>(loc, in, n, p.coarse_log, p.C, cfill, pa,
-                                 vec_loc && (!kScatter || vec_in), st);
+  s = launch_partition<true>(loc, in, n, p.coarse_log, p.C, cfill, pa, vec_loc && aligned16(in), st);
   if (s != EDPP_OK) return s;
   unsigned *fault = fault_word();
   if (!fault) return EDPP_ECUDA;
   const int64_t rblocks = static_cast<int64_t>(sms) * kRefineBlocksPerSm;
   win_refine_kernel<<<static_cast<unsigned>(min64(tiles, rblocks)), kThreads, refine_smem(), st>>>(
-      pa, start + p.F, nullptr, 0, p.fine_log, p.coarse_log, tiles, fill, pb_off, pb_val,
-      kDefaultWaitNs, fault);
-  if (kScatter) {
-    win_apply_kernel<<<static_cast<unsigned>(p.F), kWinThreads, apply_smem(p.fine_log), st>>>(
-        pb_off, pb_val, start, nullptr, p.fine_log, n, out, aligned16(out), false);
-  } else {
-    win_fetch_kernel<<<static_cast<unsigned>(p.F), kFetchThreads, fetch_smem(p.fine_log, p.C), st>>>(
-        pb_off, pb_val, start, in, n, p.fine_log, p.coarse_log, p.C, cfill2, pa, vec_in,
-        kDefaultWaitNs, fault);
-    const int64_t rtiles = static_cast<int64_t>(p.C) << (p.coarse_log - 12);
-    win_refine_kernel<<<static_cast<unsigned>(min64(rtiles, rblocks)), kThreads, refine_smem(), st>>>(
-        pa, nullptr, cfill2, p.coarse_log, p.fine_log, p.coarse_log, rtiles, fill2, pb_off, pb_val,
-        kDefaultWaitNs, fault);
-    win_apply_kernel<<<static_cast<unsigned>(p.F), kWinThreads, apply_smem(p.fine_log), st>>>(
-        pb_off, pb_val, nullptr, fill2, p.fine_log, n, out, aligned16(out), true);
-  }
+      pa, start + p.F, p.fine_log, p.coarse_log, tiles, fill, pb_off, pb_val, kDefaultWaitNs, fault);
+  win_apply_kernel<<<static_cast<unsigned>(p.F), kWinThreads, apply_smem(p.fine_log), st>>>(
+      pb_off, pb_val, start, p.fine_log, n, out, aligned16(out));
   return launch_status();
+}
+
+// Argument checks shared by the tiled entry points; EDPP_OK with n > 0 means run.
+int tiled_args(const int32_t *in, const int32_t *out, int64_t n, const int32_t *loc, int pass) {
+  if (n < 0 || pass < 0) return EDPP_EINVAL;
+  if (n == 0) return EDPP_OK;
+  if (!in || !out || !loc) return EDPP_EINVAL;
+  if (n > INT32_MAX) return EDPP_EINVAL;
+  return EDPP_OK;
 }
 
 }  // namespace
@@ -1313,33 +1174,37 @@ int edpp_scatter_i32_ws(const int32_t *in, int32_t *out, int64_t length, const i
 
 size_t edpp_gather_tiled_workspace_size(int64_t length) {
   if (length <= 0) return 0;
-  if (!edpp::tiled_fits(length)) return edpp_gather_workspace_size(length, 0);
-  return edpp::tlayout_of(length, edpp::tplan(length), true).bytes;
+  // never smaller than the scatter's, so one workspace can serve both
+  return std::max(edpp::gather_tiled_bytes(length), edpp_scatter_tiled_workspace_size(length));
 }
 
 size_t edpp_scatter_tiled_workspace_size(int64_t length) {
   if (length <= 0) return 0;
   if (!edpp::tiled_fits(length)) return edpp_scatter_workspace_size(length, 0);
-  return edpp::tlayout_of(length, edpp::tplan(length), false).bytes;
+  return edpp::tlayout_of(length, edpp::tplan(length)).bytes;
 }
 
 int edpp_gather_i32_tiled(const int32_t *in, int32_t *out, int64_t length, const int32_t *loc,
                           int pass, void *ws, size_t ws_bytes, void *stream) {
-  return edpp::tiled_run<false>(in, out, length, loc, pass, ws, ws_bytes, stream);
+  const int s = edpp::tiled_args(in, out, length, loc, pass);
+  if (s != EDPP_OK || length == 0) return s;
+  return edpp::gather_tiled(in, out, length, loc, ws, ws_bytes, edpp::as_stream(stream));
 }
 
 int edpp_scatter_i32_tiled(const int32_t *in, int32_t *out, int64_t length, const int32_t *loc,
                            int pass, void *ws, size_t ws_bytes, void *stream) {
-  return edpp::tiled_run<true>(in, out, length, loc, pass, ws, ws_bytes, stream);
+  const int s = edpp::tiled_args(in, out, length, loc, pass);
+  if (s != EDPP_OK || length == 0) return s;
+  return edpp::scatter_tiled(in, out, length, loc, ws, ws_bytes, stream);
 }
 
 int edpp_gather_prefers_direct(int64_t length) {
-  // Without a tuning entry: a gather whose source is at most ~2.5x L2 keeps
-  // enough of it in L2 that the direct random sweep wins (measured, int32
-  // permutations: 2^25 0.49 ms direct against 0.59 ms tiled; 2^26 1.00
-  // against 1.10; 2^28 5.34 against 4.32).
+  // Without a tuning entry: while the source fits L2 its random reads are
+  // served from there and the direct sweep wins (int32 permutations, direct
+  // against tiled: 2^24 0.073 against 0.149 ms; 2^25, just over L2, 0.308
+  // against 0.277; 2^26 1.00 against 0.54).
   const bool rule =
-      static_cast<double>(length) * 4.0 <= 2.5 * static_cast<double>(edpp::device_l2_bytes());
+      static_cast<double>(length) * 4.0 <= 0.9 * static_cast<double>(edpp::device_l2_bytes());
   return edpp::tuned_variant(EDPP_TUNE_GATHER, 4, length, rule ? 1 : 0) == 1;
 }
 

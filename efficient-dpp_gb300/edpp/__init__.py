@@ -283,8 +283,8 @@ def gs_workspace_bytes(kind: str, n: int, passes: int, method: str = "partition"
 def gather(inp, loc, passes: int = 1, out=None, method: str = "sweep", ws=None):
     """out[i] = inp[loc[i]].  method "sweep": one launch per pass window, each
     reading all of loc (the reference's schedule); "partition": the windows
-    as partitions (passes=0 sizes them to L2); "tiled": shared-memory
-    windows; "auto": the faster of the single direct sweep and "tiled" for
+    as partitions (passes=0 sizes them to L2); "tiled": windows
+    inside tiles; "auto": the faster of the single direct sweep and "tiled" for
     this size (the result does not depend on passes or method)."""
     return _gs("gather", inp, loc, passes, out, method, ws)
 

@@ -137,13 +137,15 @@ int edpp_scatter_i32_ws(const int32_t *in, int32_t *out, int64_t length,
                         const int32_t *loc, int pass, void *ws, size_t ws_bytes,
                         void *stream);
 
-/* Shared-memory-window gather / scatter: the same results again, for every
- * pass count (pass >= 0 is accepted for the same signature; the windows are
- * fixed by shared memory, 2^14 or 2^15 elements).  Requests are partitioned
- * twice by window (128 coarse windows, then fine windows) and one block per
- * fine window serves them inside a shared-memory copy of that window, so no
- * global access is random.  length <= 2^29; longer arrays take the
- * L2-window path (pass 0) with the workspace sized for it. */
+/* Tiled gather / scatter: the same results again, for every pass count
+ * (pass >= 0 is accepted for the same signature; the windows are fixed by
+ * L2 and shared memory).  The gather groups its requests by L2-sized window
+ * inside tiles of 8192 and reads each window while it sits in L2.  The
+ * scatter partitions its pairs twice by window (128 coarse windows, then
+ * fine windows of 2^14 or 2^15 elements) and one block per fine window
+ * serves them inside a shared-memory copy of that window; above 2^29
+ * elements it takes the L2-window path (pass 0).  The gather's workspace is
+ * never smaller than the scatter's. */
 size_t edpp_gather_tiled_workspace_size(int64_t length);
 size_t edpp_scatter_tiled_workspace_size(int64_t length);
 int edpp_gather_i32_tiled(const int32_t *in, int32_t *out, int64_t length,
@@ -155,8 +157,7 @@ int edpp_scatter_i32_tiled(const int32_t *in, int32_t *out, int64_t length,
 /* 1 when a gather of `length` elements is faster as the direct single sweep
  * (edpp_gather_i32, pass 1) than in the tiled form on the current device.
  * The tuning table's choice for this size class when it has one
- * (EDPP_TUNE_GATHER), else the rule that the source is small enough (about
- * 2.5x L2) to stay largely in L2.  Scatter always favours the tiled form. */
+ * (EDPP_TUNE_GATHER), else whether the source fits L2.  Scatter always favours the tiled form. */
 int edpp_gather_prefers_direct(int64_t length);
 
 /* ---- global scan -------------------------------------------------------- */
