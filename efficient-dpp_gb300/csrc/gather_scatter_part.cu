@@ -1208,4 +1208,13 @@ int edpp_gather_prefers_direct(int64_t length) {
   return edpp::tuned_variant(EDPP_TUNE_GATHER, 4, length, rule ? 1 : 0) == 1;
 }
 
+int edpp_scatter_prefers_direct(int64_t length) {
+  // One launch instead of six, and random 4-byte stores that run at L2's rate
+  // while most of the destination fits there (int32 permutations, direct
+  // against tiled, device time: 10^5 0.011 against 0.034 ms; 2^24 0.086
+  // against 0.170; 2.4e7 0.181 against 0.230; 2.8e7 0.266 against 0.262; 2^25
+  // 0.564 against 0.305).
+  return static_cast<double>(length) * 4.0 <= 0.8 * static_cast<double>(edpp::device_l2_bytes());
+}
+
 }  // extern "C"

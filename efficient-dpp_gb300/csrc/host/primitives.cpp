@@ -82,6 +82,8 @@ double gather(const int *d_in, int *d_out, int length, const int *d_loc, int, in
 
 double scatter(const int *d_in, int *d_out, int length, const int *d_loc, int, int, int pass) {
   if (pass < 1) return -1;
+  if (edpp_scatter_prefers_direct(length))  // the destination stays in L2
+    return timed([&] { return edpp_scatter_i32(d_in, d_out, length, d_loc, 1, nullptr); });
   Temp ws(edpp_scatter_tiled_workspace_size(length));
   if (!ws.ok()) return -1;
   return timed([&] {

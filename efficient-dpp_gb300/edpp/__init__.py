@@ -68,6 +68,7 @@ SIGNATURES = {
     "edpp_cache_heat_i32": (_I, [_VP, _I64, _I, _I, _VP]),
     "edpp_local_scan_i32": (_I, [_VP, _VP, _I, _I, _I, _VP]),
     "edpp_gather_prefers_direct": (_I, [_I64]),
+    "edpp_scatter_prefers_direct": (_I, [_I64]),
     "edpp_gather_tiled_workspace_size": (_SZ, [_I64]),
     "edpp_scatter_tiled_workspace_size": (_SZ, [_I64]),
     "edpp_gather_i32_tiled": (_I, [_VP, _VP, _I64, _VP, _I, _VP, _SZ, _VP]),
@@ -203,8 +204,9 @@ def _gs(kind, inp, loc, passes, out, method, ws):
         out = torch.zeros(n, dtype=torch.int32, device=loc.device)
     st = current_stream_handle()
     if method == "auto":  # the faster schedule for this size
-        method = ("sweep" if kind == "gather" and lib().edpp_gather_prefers_direct(n)
-                  else "tiled")
+        direct = (lib().edpp_gather_prefers_direct if kind == "gather"
+                  else lib().edpp_scatter_prefers_direct)
+        method = "sweep" if direct(n) else "tiled"
         passes = 1 if method == "sweep" else passes
     if method == "sweep":
         f = lib().edpp_gather_i32 if kind == "gather" else lib().edpp_scatter_i32

@@ -154,11 +154,13 @@ int edpp_gather_i32_tiled(const int32_t *in, int32_t *out, int64_t length,
 int edpp_scatter_i32_tiled(const int32_t *in, int32_t *out, int64_t length,
                            const int32_t *loc, int pass, void *ws, size_t ws_bytes,
                            void *stream);
-/* 1 when a gather of `length` elements is faster as the direct single sweep
- * (edpp_gather_i32, pass 1) than in the tiled form on the current device.
- * The tuning table's choice for this size class when it has one
- * (EDPP_TUNE_GATHER), else whether the source fits L2.  Scatter always favours the tiled form. */
+/* 1 when a gather (scatter) of `length` elements is faster as the direct
+ * single sweep (edpp_gather_i32 / edpp_scatter_i32, pass 1) than in the tiled
+ * form on the current device.  Gather: the tuning table's choice for this
+ * size class when it has one (EDPP_TUNE_GATHER), else whether the source fits
+ * L2.  Scatter: whether the destination fits 80% of L2. */
 int edpp_gather_prefers_direct(int64_t length);
+int edpp_scatter_prefers_direct(int64_t length);
 
 /* ---- global scan -------------------------------------------------------- */
 
