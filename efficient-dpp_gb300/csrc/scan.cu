@@ -11,9 +11,12 @@
 //            synchronisation (opencl/primitives/scanImpl.cpp:15-66,
 //            opencl/kernels/scan_global_chain_kernel.cl:11-203), whose
 //            tile t waits for tile t-1 only and spins without a limit.
-//  RTS       reduce-then-scan in three launches (per-block reduction, scan of
-//            the block sums in one block, per-block rescan with the offset):
-//            traffic 3n.  The reference's RSS scan
+//  RTS       reduce-then-scan: a tile's sum is published before the tile is
+//            scanned.  One cooperative launch that keeps the tile in shared
+//            memory (scan_pipe.cu) or in L2 (rts_fused, rts_chunked) between
+//            its two reads: traffic 2n; where no cooperative grid fits, three
+//            launches (per-block reduction, scan of the block sums in one
+//            block, per-block rescan with the offset): traffic 3n.  The reference's RSS scan
 //            (opencl/primitives/scanImpl.cpp:69-160,
 //            opencl/kernels/scan_global_RSS_kernel.cl:142-240) and
 //            scan_RTS_omp (openmp/test_scan_CPU.cpp:125-163).
@@ -27,6 +30,7 @@
 #include <algorithm>
 #include <mutex>
 
+#include "scan_pipe.h"
 #include "scan_tile.cuh"
 #include "tune.h"
 
@@ -51,8 +55,8 @@ template <typename T> using TS = TileScan<T, kThreads, kChunks>;
 //   variant 1  256 x 8   32 KB tiles,  6 / 4 blocks per SM (half the tiles,
 //              so half the look-backs)
 //   variant 2  512 x 4   32 KB tiles,  6 / 4 blocks per SM
-//   variant 3  512 x 8   64 KB tiles,  3 / 2 blocks per SM (a quarter of the
-//              look-backs)
+//   variant 3  the pipelined one-launch scan (scan_pipe.cu) for 16-byte
+//              aligned arrays; variant 1 otherwise
 // Variant 0's tiles are the smallest; tile state and workspace are sized
 // for them, so every shape fits the same workspace.
 constexpr int kLbThreads = 128;
@@ -377,7 +381,8 @@ __global__ void __launch_bounds__(kThreads)
 // bounded; a block that gives up raises EDPP_FAULT_TIMEOUT and sets the
 // call's abort flag so the others stop too.
 // kSliceTiles is the slice length in tiles, chosen per size class by the
-// tuning table: variant 0 two tiles (the default), variant 1 one tile,
+// tuning table: variant 0 (the default) two tiles, for arrays off 16-byte
+// alignment only (others take the pipelined scan_pipe.cu), variant 1 one tile,
 // variant 2 four tiles (reduced in two rounds of eight 16-byte loads per
 // thread), variant 3 two tiles with L2 eviction hints (kHint: the reduce's
 // loads evict-last, the second read's bulk copies evict-first), variant 4
@@ -563,7 +568,7 @@ template <typename T> size_t workspace_bytes(int64_t n, int algo) {
   if (algo != EDPP_SCAN_RTS) return three;
   const size_t chunked = kHeader + chunked_sums_bytes<T>(n) +
                          round_up(static_cast<size_t>(slices_of<T>(n)) * 4, 256);
-  return std::max(three, chunked);
+  return std::max({three, chunked, kHeader + scan_pipe_state_bytes<T>(n)});
 }
 
 // Blocks of the RTS / SSA schemes: a few waves of resident blocks, each
@@ -671,9 +676,13 @@ int scan_impl(const T *in, T *out, int64_t n, int algo, void *ws, size_t ws_byte
       case 2:
         return launch_lookback<T, kInclusive, 512, 4, 6, 4>(in, out, n, w, st, tile_base, tma,
                                                             vec_out, timeout_ns, fault);
-      case 3:
-        return launch_lookback<T, kInclusive, 512, 8, 3, 2>(in, out, n, w, st, tile_base, tma,
+      case 3: {
+        const int s = tma && vec_out ? scan_pipe<T, kInclusive>(in, out, n, w, st, timeout_ns, fault)
+                                     : EDPP_ENOMEM;
+        if (s != EDPP_ENOMEM) return s;
+        return launch_lookback<T, kInclusive, 256, 8, 6, 4>(in, out, n, w, st, tile_base, tma,
                                                             vec_out, timeout_ns, fault);
+      }
       default:
         return launch_lookback<T, kInclusive, kLbThreads, kLbChunks, 12, 8>(
             in, out, n, w, st, tile_base, tma, vec_out, timeout_ns, fault);
@@ -686,6 +695,10 @@ int scan_impl(const T *in, T *out, int64_t n, int algo, void *ws, size_t ws_byte
   const int64_t per = tpb * TS<T>::kTile;
   if (algo == EDPP_SCAN_RTS && variant < 0)
     variant = tuned_variant(EDPP_TUNE_SCAN_RTS, sizeof(T), n, 0);
+  if (algo == EDPP_SCAN_RTS && variant == 0 && tma && vec_out) {
+    const int s = scan_pipe<T, kInclusive>(in, out, n, w, st, timeout_ns, fault);
+    if (s != EDPP_ENOMEM) return s;
+  }
   if (algo == EDPP_SCAN_RTS && variant != 4 &&
       static_cast<double>(n) * sizeof(T) <= 0.6 * static_cast<double>(device_l2_bytes())) {
     // the input stays in L2 between the reduce and the scan: one launch

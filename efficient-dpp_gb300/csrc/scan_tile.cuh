@@ -25,6 +25,7 @@ __device__ __forceinline__ int64_t op_add(int64_t a, int64_t b) {
   return static_cast<int64_t>(static_cast<uint64_t>(a) + static_cast<uint64_t>(b));
 }
 __device__ __forceinline__ float op_add(float a, float b) { return a + b; }
+__device__ __forceinline__ double op_add(double a, double b) { return a + b; }
 
 template <typename T> __device__ __forceinline__ T zero_of() { return T(0); }
 

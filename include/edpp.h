@@ -484,13 +484,16 @@ void edpp_server_destroy(edpp_server *server);
  * tunables per device by hand (R, L, local and grid sizes of scan_chained,
  * opencl/test/test_scan_global.cpp:87-94); here they are measured.
  *   EDPP_TUNE_SCAN_LOOKBACK  look-back tile shape (threads x 16-byte chunks):
- *                            0 128x8 (16 KB), 1 256x8 (32 KB), 2 512x4 (32 KB),
- *                            3 512x8 (64 KB)
- *   EDPP_TUNE_SCAN_RTS       slice of the chunked reduce-then-scan (inputs
- *                            larger than 60% of L2): 0 two tiles, 1 one,
- *                            2 four, 3 two with L2 eviction hints (first read
- *                            kept, second read demoted), 4 two tiles and the
- *                            chunked form also below 60% of L2
+ *                            0 128x8 (16 KB), 1 256x8 (32 KB), 2 512x4 (32 KB);
+ *                            3 the pipelined one-launch scan (variant 1 for
+ *                            arrays off 16-byte alignment)
+ *   EDPP_TUNE_SCAN_RTS       0 the pipelined one-launch scan (arrays off 16-byte
+ *                            alignment: slices of two tiles); else the slice
+ *                            of the chunked reduce-then-scan (inputs larger
+ *                            than 60% of L2): 1 one tile, 2 four, 3 two with
+ *                            L2 eviction hints (first read kept, second read
+ *                            demoted), 4 two tiles and the chunked form also
+ *                            below 60% of L2
  *   EDPP_TUNE_GATHER         0 tiled form, 1 direct single sweep (the choice
  *                            edpp_gather_prefers_direct reports)
  * The table is read from efficient-dpp_gb300/tuning/plain_gb300.tsv (beside
