@@ -25,11 +25,16 @@
 //              in bucket order, and written out as one contiguous run per
 //              bucket (coalesced), at his[b*T + t] + rank.
 //
+// Inputs whose tiles are all resident at once (up to 2.4 million elements) take
+// one cooperative launch instead (the fused form of the scatter kernel): the
+// tile is read once, its counts come from its ranking, and the blocks exchange
+// them through his.
+//
 // Ranks follow input order inside a warp segment, warp segments follow
 // input order inside a tile, tiles follow input order in the scan: the split
 // is stable, bit-identical to single_split (split_kernel.cl:676-736),
-// WG_split with FIXED_REORDER and the CUDA pre_scan/post_scan split.  There
-// are no inter-block waits.
+// WG_split with FIXED_REORDER and the CUDA pre_scan/post_scan split.  Only
+// the fused form waits between blocks (once, bounded).
 #include <algorithm>
 #include <mutex>
 
@@ -111,10 +116,11 @@ __global__ void __launch_bounds__(kHistThreads)
 }
 
 // ---- stage 3: stable scatter --------------------------------------------------
-template <int THREADS> struct ScatterCfg {
+// TILE elements per block.
+template <int THREADS, int TILE = kTile> struct ScatterCfg {
   static constexpr int kWarps = THREADS / 32;
-  static constexpr int kSeg = kTile / kWarps;  // elements per warp
-  static constexpr int kIters = kSeg / 32;     // per lane
+  static constexpr int kSeg = TILE / kWarps;  // elements per warp
+  static constexpr int kIters = kSeg / 32;    // per lane
 };
 
 // Bucket runs written by bulk copies (KO and KVS_SOA, 3 to kBulkBuckets
@@ -125,8 +131,8 @@ template <int THREADS> struct ScatterCfg {
 // both builds): 4 / 8 / 16 buckets 9 / 7 / 4% faster; from 32 buckets on,
 // with runs of 256 elements or fewer, 3-14% slower.
 constexpr int kBulkBuckets = 16;
-__host__ __device__ constexpr int stage_len(int buckets, bool bulk) {
-  return kTile + (bulk ? (3 * buckets + 3) / 4 * 4 : 0);
+__host__ __device__ constexpr int stage_len(int tile, int buckets, bool bulk) {
+  return tile + (bulk ? (3 * buckets + 3) / 4 * 4 : 0);
 }
 
 // Peer table of the ranking, per warp: from kRegBits + 1 to 8 bucket bits one
@@ -137,10 +143,10 @@ __host__ __device__ constexpr int peer_table_bytes(int buckets) {
 }
 
 // Dynamic shared memory of the scatter kernel.
-template <int THREADS, int LAYOUT> size_t scatter_smem_bytes(int buckets, bool bulk = false) {
-  const size_t stage = (LAYOUT == EDPP_KO) ? 4 * static_cast<size_t>(stage_len(buckets, bulk))
-                       : (LAYOUT == EDPP_KVS_SOA) ? 8 * static_cast<size_t>(stage_len(buckets, bulk))
-                                                  : kTile * 8;
+template <int THREADS, int LAYOUT, int TILE = kTile>
+size_t scatter_smem_bytes(int buckets, bool bulk = false) {
+  const size_t len = static_cast<size_t>(stage_len(TILE, buckets, bulk));
+  const size_t stage = LAYOUT == EDPP_KO ? 4 * len : LAYOUT == EDPP_KVS_SOA ? 8 * len : TILE * 8;
   return stage + round_up(static_cast<size_t>(ScatterCfg<THREADS>::kWarps) * buckets * 2, 16) +
          2 * static_cast<size_t>(buckets) * 4 +
          static_cast<size_t>(ScatterCfg<THREADS>::kWarps) * peer_table_bytes(buckets);
@@ -152,24 +158,125 @@ template <int THREADS, int LAYOUT> size_t scatter_smem_bytes(int buckets, bool b
 // carrying every form: 16 / 32 / 64 / 256 buckets 19 / 14 / 12 / 7% faster
 // at 2^28 pairs, 512 and 1024 even (one process, both builds).  A third
 // kernel for the register counts alone spilled and made 2 buckets 4% slower.
-template <int THREADS, int LAYOUT, bool kWide>
+//
+// kFused: the whole split in one cooperative launch, for inputs whose tiles are
+// all resident together.  The tile's bucket counts come from its own ranking;
+// they are published as row t of his, and once every block has arrived at
+// *fused.arrived (bounded wait) each block adds up what precedes its runs: the
+// smaller buckets' totals and its bucket's counts in the tiles before.  The
+// tile waits in registers meanwhile.
+struct FusedArgs {
+  unsigned *arrived;      // zeroed before the launch
+  int32_t *his;           // [tiles][buckets]
+  int32_t *bucket_start;  // may be null
+};
+
+// Output start of every bucket's run of tile t, into start[] (shared): publish
+// the tile's counts (cnt[], shared) as row t of his, wait for all tiles', add up
+// the rows.  A thread reads 16-byte quads 2048 words apart, which hold the same
+// buckets each time (the bucket counts divide 2048); tot[] is shared scratch.
+// False: the wait ran out.
+template <int THREADS>
+__device__ __forceinline__ bool fused_starts(const FusedArgs &f, int t, int tiles, int buckets,
+                                             const int32_t *cnt, int32_t *start, int32_t *tot,
+                                             uint64_t timeout_ns, unsigned *fault) {
+  static_assert(2048 % (4 * THREADS) == 0, "a thread's quads hold the same buckets");
+  constexpr int kWarps = THREADS / 32;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  __shared__ int32_t s_sum[kWarps];
+  __shared__ int s_ok;
+  for (int b = tid; b < buckets; b += THREADS) {
+    f.his[t * buckets + b] = cnt[b];
+    start[b] = 0;
+    tot[b] = 0;
+  }
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) {
+    atomicAdd(f.arrived, 1u);
+    const uint64_t t0 = globaltimer_ns();
+    bool ok;
+    while (!(ok = ld_acquire_u32(f.arrived) >= static_cast<uint32_t>(tiles)) &&
+           globaltimer_ns() - t0 <= timeout_ns) {
+    }
+    if (!ok) raise_fault(fault, EDPP_FAULT_TIMEOUT);
+    s_ok = ok ? 1 : 0;
+  }
+  __syncthreads();
+  if (!s_ok) return false;
+  const int words = tiles * buckets, mine = t * buckets;
+  int32_t total[4] = {0, 0, 0, 0}, before[4] = {0, 0, 0, 0};
+#pragma unroll 8
+  for (int i = 4 * tid; i < words; i += 4 * THREADS) {
+    const int4 q = __ldcg(reinterpret_cast<const int4 *>(f.his + i));
+    const int32_t c[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      if (i + e < words) total[e] += c[e];
+      if (i + e < mine) before[e] += c[e];
+    }
+  }
+  // lanes whose quads hold the same buckets join before the shared atomics
+  const int quads = max(1, buckets / 4);
+  for (int m = 16; m >= quads; m >>= 1) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      total[e] += __shfl_xor_sync(0xffffffffu, total[e], m);
+      before[e] += __shfl_xor_sync(0xffffffffu, before[e], m);
+    }
+  }
+  if (lane < quads) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int b = (4 * tid + e) & (buckets - 1);
+      if (total[e]) atomicAdd(&tot[b], total[e]);
+      if (before[e]) atomicAdd(&start[b], before[e]);
+    }
+  }
+  __syncthreads();
+  // exclusive scan of the totals, thread-consecutive buckets
+  const int per = (buckets + THREADS - 1) / THREADS;
+  const int lo = min(buckets, tid * per), hi = min(buckets, lo + per);
+  int32_t sum = 0;
+  for (int b = lo; b < hi; ++b) sum += tot[b];
+  int32_t incl = sum;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int32_t y = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += y;
+  }
+  if (lane == 31) s_sum[w] = incl;
+  __syncthreads();
+  int32_t run = incl - sum;
+#pragma unroll
+  for (int k = 0; k < kWarps; ++k)
+    if (k < w) run += s_sum[k];
+  for (int b = lo; b < hi; ++b) {
+    start[b] += run;
+    run += tot[b];
+    if (t == 0 && f.bucket_start) f.bucket_start[b] = start[b];  // tile 0 starts each bucket
+  }
+  return true;
+}
+
+template <int THREADS, int LAYOUT, bool kWide, int TILE = kTile, bool kFused = false>
 __global__ void __launch_bounds__(THREADS, 2)
     split_scatter_kernel(const int32_t *__restrict__ keys_in, int32_t *__restrict__ keys_out,
                          const int32_t *__restrict__ vals_in, int32_t *__restrict__ vals_out,
                          int64_t n, int buckets, int shift, int64_t tiles,
                          const int32_t *__restrict__ his, bool tma, bool bulk,
-                         uint64_t timeout_ns, unsigned *fault) {
-  using C = ScatterCfg<THREADS>;
+                         uint64_t timeout_ns, unsigned *fault, FusedArgs fused) {
+  using C = ScatterCfg<THREADS, TILE>;
   extern __shared__ __align__(128) unsigned char smem[];
-  // Layout: stage (keys[L] + vals[L] with L = stage_len, or pairs[kTile]) |
+  // Layout: stage (keys[L] + vals[L] with L = stage_len, or pairs[TILE]) |
   // cnt16 | toff | gofs | peer tables.  `bulk` (KO / SOA only): runs go out by
   // bulk copies.
-  const int slen = stage_len(buckets, bulk);
+  const int slen = stage_len(TILE, buckets, bulk);
   int32_t *s_keys = reinterpret_cast<int32_t *>(smem);
   int32_t *s_vals = s_keys + slen;  // SOA only
   int2 *s_pairs = reinterpret_cast<int2 *>(smem);  // AOS only
   const size_t stage = LAYOUT == EDPP_KO ? 4 * static_cast<size_t>(slen)
-                       : LAYOUT == EDPP_KVS_SOA ? 8 * static_cast<size_t>(slen) : kTile * 8;
+                       : LAYOUT == EDPP_KVS_SOA ? 8 * static_cast<size_t>(slen) : TILE * 8;
   uint16_t *cnt16 = reinterpret_cast<uint16_t *>(smem + stage);
   int32_t *toff = reinterpret_cast<int32_t *>(
       smem + stage + round_up(static_cast<size_t>(C::kWarps) * buckets * 2, 16));
@@ -178,8 +285,8 @@ __global__ void __launch_bounds__(THREADS, 2)
   __shared__ alignas(8) uint64_t bar;
 
   const int64_t t = blockIdx.x;
-  const int64_t base = t * kTile;
-  const int count = static_cast<int>(min64(kTile, n - base));
+  const int64_t base = t * TILE;
+  const int count = static_cast<int>(min64(TILE, n - base));
   const unsigned mask = static_cast<unsigned>(buckets - 1);
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
 
@@ -225,7 +332,7 @@ __global__ void __launch_bounds__(THREADS, 2)
   int32_t his_pre[kHisPre];
 #pragma unroll
   for (int k = 0; k < kHisPre; ++k)
-    his_pre[k] = b_lo + k < b_hi ? __ldg(his + static_cast<int64_t>(b_lo + k) * tiles + t) : 0;
+    his_pre[k] = !kFused && b_lo + k < b_hi ? __ldg(his + static_cast<int64_t>(b_lo + k) * tiles + t) : 0;
   if (bulk_elems) {
     if (!mbar_wait_bounded(&bar, 0, timeout_ns, fault)) return;
   }
@@ -316,7 +423,7 @@ __global__ void __launch_bounds__(THREADS, 2)
   // Thread-consecutive buckets so the block-wide scan over buckets is a
   // per-thread serial scan plus one warp/ block combine.  cnt16[w][b]
   // becomes the tile slot of warp w's first element of bucket b (the
-  // bucket's tile offset plus the counts of the warps before w; < kTile, so
+  // bucket's tile offset plus the counts of the warps before w; < TILE, so
   // it fits 16 bits), which leaves the re-layout one lookup per element.
   int32_t my_total = 0;
   for (int b = b_lo; b < b_hi; ++b) {
@@ -348,6 +455,14 @@ __global__ void __launch_bounds__(THREADS, 2)
   }
   __syncthreads();
   int32_t run = s_wsum[w] + (incl - my_total);
+  if (kFused) {
+    // the staging area is free until the re-layout
+    if (!fused_starts<THREADS>(fused, static_cast<int>(t), static_cast<int>(tiles), buckets, toff,
+                               gofs, reinterpret_cast<int32_t *>(smem), timeout_ns, fault))
+      return;
+#pragma unroll
+    for (int k = 0; k < kHisPre; ++k) his_pre[k] = b_lo + k < b_hi ? gofs[b_lo + k] : 0;
+  }
   auto warp_slots = [&](int b, int32_t start) {
 #pragma unroll 4
     for (int ww = 0; ww < C::kWarps; ++ww) {
@@ -523,12 +638,96 @@ int launch_scatter(const int32_t *keys_in, int32_t *keys_out, const int32_t *val
   if (wide)
     split_scatter_kernel<THREADS, LAYOUT, true><<<grid, THREADS, smem, st>>>(
         keys_in, keys_out, vals_in, vals_out, n, buckets, shift, tiles, his, tma, bulk,
-        kDefaultWaitNs, fault_word());
+        kDefaultWaitNs, fault_word(), FusedArgs{});
   else
     split_scatter_kernel<THREADS, LAYOUT, false><<<grid, THREADS, smem, st>>>(
         keys_in, keys_out, vals_in, vals_out, n, buckets, shift, tiles, his, tma, bulk,
-        kDefaultWaitNs, fault_word());
+        kDefaultWaitNs, fault_word(), FusedArgs{});
   return launch_status();
+}
+
+// The fused split with tiles of TILE elements; EDPP_ENOMEM (nothing launched)
+// when the tiles cannot all be resident or the cooperative launch is refused.
+template <int LAYOUT, bool kWide, int TILE>
+int launch_fused(const int32_t *keys_in, int32_t *keys_out, const int32_t *vals_in,
+                 int32_t *vals_out, int32_t *bucket_start, int64_t n, int buckets, int shift,
+                 char *ws, bool tma, cudaStream_t st) {
+  constexpr int THREADS = 512;
+  auto *kernel = split_scatter_kernel<THREADS, LAYOUT, kWide, TILE, true>;
+  static std::once_flag once[64];
+  static int resident[64];  // of the largest bucket count
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) dev = 0;
+  std::call_once(once[dev], [dev, kernel] {
+    const size_t bytes = scatter_smem_bytes<THREADS, LAYOUT, TILE>(kWide ? kOnePassMax : 256, true);
+    int per_sm = 0;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             static_cast<int>(bytes)) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, THREADS, bytes) !=
+            cudaSuccess) {
+      per_sm = 0;
+      cudaGetLastError();
+    }
+    resident[dev] = per_sm * device_sm_count();
+  });
+  int64_t tiles = (n + TILE - 1) / TILE;
+  if (tiles > resident[dev]) return EDPP_ENOMEM;
+  bool bulk = LAYOUT != EDPP_KVS_AOS && buckets > kDirectBuckets && buckets <= kBulkBuckets &&
+              aligned16(keys_out) && (LAYOUT != EDPP_KVS_SOA || aligned16(vals_out));
+  const size_t smem = scatter_smem_bytes<THREADS, LAYOUT, TILE>(buckets, bulk);
+  if (cudaMemsetAsync(ws, 0, 16, st) != cudaSuccess) return EDPP_ECUDA;
+  int32_t *his = reinterpret_cast<int32_t *>(ws + 256);
+  FusedArgs fused{reinterpret_cast<unsigned *>(ws), his, bucket_start};
+  uint64_t timeout_ns = kDefaultWaitNs;
+  unsigned *fault = fault_word();
+  void *args[] = {&keys_in, &keys_out, &vals_in, &vals_out, &n,    &buckets,    &shift, &tiles,
+                  &his,     &tma,      &bulk,    &timeout_ns, &fault, &fused};
+  if (cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(kernel),
+                                  dim3(static_cast<unsigned>(tiles)), dim3(THREADS), args, smem,
+                                  st) != cudaSuccess) {
+    cudaGetLastError();
+    return EDPP_ENOMEM;
+  }
+  return launch_status();
+}
+
+// The fused form takes an input when its tiles are all resident (two blocks per
+// SM) and the words every block adds up are few: device time, three launches
+// against fused, key/value pairs: 256 buckets 10^5 pairs 20.6 -> 12.7 us, 10^6
+// 22.0 -> 18.9, 2*10^6 (62720 words) 28.0 -> 28.5, the line; 1024 buckets
+// 3*10^5 28.6 -> 22.6, and past the line 10^6 26.4 -> 28.8.  The smallest tile
+// that still leaves one block per SM: 6*10^5 pairs, 256 buckets, 4096-pair tiles
+// 14.4 us, 2048 (two blocks per SM) 17.0; 10^6 pairs 8192-pair tiles 18.9, 4096
+// 20.6.
+constexpr int64_t kFusedWords = 1 << 16;
+constexpr int kSmallTile = 2048, kMidTile = 4096;
+
+// Workspace of the fused form (256 bytes for the counter, then his), an upper
+// bound over its tile sizes.
+size_t fused_ws_bytes(int64_t n, int buckets) {
+  return 256 + 4 * static_cast<size_t>(min64(kFusedWords, (n + kSmallTile - 1) / kSmallTile * buckets));
+}
+
+template <int LAYOUT, bool kWide>
+int split_fused(const int32_t *keys_in, int32_t *keys_out, const int32_t *vals_in,
+                int32_t *vals_out, int32_t *bucket_start, int64_t n, int buckets, int shift,
+                char *ws, bool tma, cudaStream_t st) {
+  const int64_t sms = device_sm_count();
+  auto fits = [&](int64_t tile, int64_t blocks) {
+    const int64_t tiles = (n + tile - 1) / tile;
+    return tiles <= blocks && tiles * buckets <= kFusedWords;
+  };
+  if (fits(kSmallTile, sms))
+    return launch_fused<LAYOUT, kWide, kSmallTile>(keys_in, keys_out, vals_in, vals_out,
+                                                   bucket_start, n, buckets, shift, ws, tma, st);
+  if (fits(kMidTile, sms))
+    return launch_fused<LAYOUT, kWide, kMidTile>(keys_in, keys_out, vals_in, vals_out,
+                                                 bucket_start, n, buckets, shift, ws, tma, st);
+  if (fits(kTile, 2 * sms))
+    return launch_fused<LAYOUT, kWide, kTile>(keys_in, keys_out, vals_in, vals_out, bucket_start,
+                                              n, buckets, shift, ws, tma, st);
+  return EDPP_ENOMEM;
 }
 
 template <int LAYOUT>
@@ -542,9 +741,13 @@ int split_layout(const int32_t *keys_in, int32_t *keys_out, int32_t *bucket_star
   void *scan_ws = static_cast<char *>(ws) + his_bytes(tiles, buckets);
   const size_t scan_ws_bytes = ws_bytes - his_bytes(tiles, buckets);
   bool tma = aligned16(keys_in) && (LAYOUT != EDPP_KVS_SOA || aligned16(vals_in));
+  int s = (buckets > 256 ? split_fused<LAYOUT, true> : split_fused<LAYOUT, false>)(
+      keys_in, keys_out, vals_in, vals_out, bucket_start, n, buckets, shift,
+      static_cast<char *>(ws), tma, st);
+  if (s != EDPP_ENOMEM) return s;
   split_hist_kernel<LAYOUT><<<static_cast<unsigned>(tiles), kHistThreads, 0, st>>>(
       keys_in, n, buckets, shift, tiles, his, aligned16(keys_in));
-  int s = launch_status();
+  s = launch_status();
   if (s != EDPP_OK) return s;
   s = edpp_scan_exclusive_i32(his, his, hlen, EDPP_SCAN_LOOKBACK, scan_ws, scan_ws_bytes, st);
   if (s != EDPP_OK) return s;
@@ -566,8 +769,9 @@ constexpr int kLsdBuckets = 2048;
 
 size_t split_pass_ws_bytes(int64_t n, int buckets) {
   const int64_t tiles = (n + kTile - 1) / kTile;
-  return his_bytes(tiles, buckets) +
-         edpp_scan_workspace_size(tiles * buckets, EDPP_I32, EDPP_SCAN_LOOKBACK);
+  return std::max(his_bytes(tiles, buckets) +
+                      edpp_scan_workspace_size(tiles * buckets, EDPP_I32, EDPP_SCAN_LOOKBACK),
+                  fused_ws_bytes(n, buckets));
 }
 
 // LSD workspace: temporary keys and values (two arrays of 4 bytes per
