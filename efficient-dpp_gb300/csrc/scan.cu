@@ -126,6 +126,107 @@ __global__ void __launch_bounds__(TH, MINB)
   S::store(out, base, count, c, vec_out);
 }
 
+// ---- small inputs: one thread-block cluster ----------------------------------
+// Up to kSmallBlocks tiles of 32 or 64 KB, one per block of a cluster: a block
+// scans its tile in registers, writes the tile's sum into the shared memory of
+// every block of the cluster, and after one cluster barrier adds up the sums
+// before its own.  No state in global memory, so no memset ahead of the launch
+// and no look-back: bound by launch and load latency.  Device time of one call
+// among others in a graph, int32: 1000 elements 6.3 -> 2.3 us, 65536 6.4 -> 3.0
+// (reduce-then-scan 8.3 -> 3.0), 131072 6.8 -> 3.8.
+constexpr int kSmallThreads = 512, kSmallBlocks = 8;
+template <typename T, int CH> using TSS = TileScan<T, kSmallThreads, CH>;
+
+// Shared-memory store into block `rank` of the cluster.
+__device__ __forceinline__ void st_cluster(void *p, unsigned rank, uint64_t bits, int bytes) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr(p)), "r"(rank));
+  if (bytes == 4)
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(static_cast<uint32_t>(bits))
+                 : "memory");
+  else
+    asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(a), "l"(bits) : "memory");
+}
+
+__device__ __forceinline__ void cluster_arrive() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <typename T, bool kInclusive, int CH>
+__global__ void __launch_bounds__(kSmallThreads)
+    scan_small_kernel(const T *in, T *out, int64_t n, bool vec_in, bool vec_out) {
+  using S = TSS<T, CH>;
+  constexpr int E = Chunk<T>::E;
+  __shared__ typename S::Shared sh;
+  __shared__ T sums[kSmallBlocks];
+  const int t = threadIdx.x, lane = t & 31;
+  const unsigned blocks = gridDim.x, b = blockIdx.x;  // one cluster: rank = block index
+  const int64_t base = static_cast<int64_t>(b) * S::kTile;
+  const int count = static_cast<int>(min64(S::kTile, n - base));
+  cluster_arrive();  // waited for before the first store into another block
+  Chunk<T> c[CH];
+#pragma unroll
+  for (int k = 0; k < CH; ++k) {
+    const int first = (k * kSmallThreads + t) * E;
+    if (vec_in && first + E <= count) {
+      c[k].raw = *reinterpret_cast<const uint4 *>(in + base + first);
+    } else {
+#pragma unroll
+      for (int e = 0; e < E; ++e) c[k].e[e] = first + e < count ? in[base + first + e] : zero_of<T>();
+    }
+  }
+  T wex[CH];
+  S::scan_chunks(c, wex, sh);
+  __syncthreads();
+  cluster_wait();
+  if (t < 32) {
+    const T agg = S::phase2_warp0(sh, lane);
+    if (static_cast<unsigned>(lane) < blocks) {
+      uint64_t bits = 0;
+      memcpy(&bits, &agg, sizeof(T));
+      st_cluster(&sums[b], lane, bits, sizeof(T));
+    }
+  }
+  __syncwarp();
+  cluster_arrive();  // all sums have arrived, and warp_pre is visible to the block
+  cluster_wait();
+  T prefix = zero_of<T>();
+#pragma unroll
+  for (unsigned r = 0; r + 1 < kSmallBlocks; ++r)
+    if (r < b) prefix = op_add(prefix, sums[r]);
+  S::template phase3<kInclusive>(c, wex, sh, prefix);
+  S::store(out, base, count, c, vec_out);
+}
+
+template <typename T, bool kInclusive, int CH>
+int launch_small_as(const T *in, T *out, int64_t n, cudaStream_t st) {
+  const unsigned blocks = static_cast<unsigned>((n + TSS<T, CH>::kTile - 1) / TSS<T, CH>::kTile);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(kSmallThreads);
+  cfg.stream = st;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = blocks;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cuda_status(cudaLaunchKernelEx(&cfg, scan_small_kernel<T, kInclusive, CH>, in, out, n,
+                                        aligned16(in), aligned16(out)));
+}
+
+// The longest input of the cluster form.
+template <typename T> constexpr int64_t small_max() { return kSmallBlocks * TSS<T, 8>::kTile; }
+
+template <typename T, bool kInclusive>
+int launch_small(const T *in, T *out, int64_t n, cudaStream_t st) {
+  return n <= kSmallBlocks * TSS<T, 4>::kTile ? launch_small_as<T, kInclusive, 4>(in, out, n, st)
+                                              : launch_small_as<T, kInclusive, 8>(in, out, n, st);
+}
+
 // ---- RTS / SSA building blocks ----------------------------------------------
 
 // Sum of in[lo, hi) by the whole block; the result is valid in thread 0.
@@ -667,6 +768,8 @@ int scan_impl(const T *in, T *out, int64_t n, int algo, void *ws, size_t ws_byte
   const bool vec_out = aligned16(out);
   char *w = static_cast<char *>(ws);
 
+  if (variant < 0 && algo != EDPP_SCAN_SSA && n <= small_max<T>())
+    return launch_small<T, kInclusive>(in, out, n, st);
   if (algo == EDPP_SCAN_LOOKBACK) {
     if (variant < 0) variant = tuned_variant(EDPP_TUNE_SCAN_LOOKBACK, sizeof(T), n, 0);
     switch (variant) {

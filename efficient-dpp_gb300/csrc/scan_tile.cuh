@@ -191,11 +191,19 @@ template <typename T, int THREADS, int CHUNKS> struct TileScan {
   // and publish warp totals.  Caller then __syncthreads().
   __device__ __forceinline__ static void phase1(const T *tile_smem, Chunk<T> (&c)[CHUNKS],
                                                 T (&warp_excl)[CHUNKS], Shared &sh) {
+#pragma unroll
+    for (int k = 0; k < CHUNKS; ++k)
+      c[k].raw = reinterpret_cast<const uint4 *>(tile_smem)[k * THREADS + threadIdx.x];
+    scan_chunks(c, warp_excl, sh);
+  }
+
+  // Phase 1 on chunks already in registers.
+  __device__ __forceinline__ static void scan_chunks(Chunk<T> (&c)[CHUNKS], T (&warp_excl)[CHUNKS],
+                                                     Shared &sh) {
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
     T incl[CHUNKS];
 #pragma unroll
     for (int k = 0; k < CHUNKS; ++k) {
-      c[k].raw = reinterpret_cast<const uint4 *>(tile_smem)[k * THREADS + t];
 #pragma unroll
       for (int e = 1; e < E; ++e) c[k].e[e] = op_add(c[k].e[e - 1], c[k].e[e]);
       incl[k] = c[k].e[E - 1];
