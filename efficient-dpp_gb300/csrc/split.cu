@@ -14,16 +14,15 @@
 //              reference runs scan_chained(d_his, d_his, ...) in place
 //              (splitImpl.cpp:97).  his[b*T + t] is then the first output
 //              index of bucket b's elements from tile t.
-//  3. scatter: one block per tile stages the tile in shared memory by TMA
+//  3. scatter: one block per tile brings the tile into shared memory by TMA
 //              bulk copy; every warp ranks its contiguous 1/WARPS of the tile
-//              in input order (rank = popc of the lower lanes in the
-//              element's peer group + the warp's running count of the
-//              bucket; the peer group from votes on the bucket bits up to 4
-//              buckets, from a per-warp lane mask per bucket up to 256, from
-//              a leader table plus votes above); ranks of all warps are
-//              combined per bucket, the tile is re-laid out in shared memory
-//              in bucket order, and written out as one contiguous run per
-//              bucket (coalesced), at his[b*T + t] + rank.
+//              in input order; ranks of all warps are combined per bucket, the
+//              tile is re-laid out in shared memory in bucket order, and
+//              written out as one contiguous run per bucket (coalesced), at
+//              his[b*T + t] + rank.  Few buckets rank by votes or per-warp lane
+//              masks and re-lay the elements out (below); from 8 to 64 buckets
+//              on, depending on the layout, one atomic per element ranks and
+//              only source positions are re-laid out (split_index.cuh).
 //
 // Inputs whose tiles are all resident at once (up to 2.4 million elements) take
 // one cooperative launch instead (the fused form of the scatter kernel): the
@@ -135,29 +134,19 @@ __host__ __device__ constexpr int stage_len(int tile, int buckets, bool bulk) {
   return tile + (bulk ? (3 * buckets + 3) / 4 * 4 : 0);
 }
 
-// Peer table of the ranking, per warp: from kRegBits + 1 to 8 bucket bits one
-// 32-bit lane mask per bucket (lanes OR themselves in); above 8 bits one
-// leader byte per value of the low 8 bucket bits.
-__host__ __device__ constexpr int peer_table_bytes(int buckets) {
-  return buckets <= 256 ? 4 * buckets : 256;
-}
-
-// Dynamic shared memory of the scatter kernel.
+// Dynamic shared memory of the scatter kernel (its peer table: per warp, one
+// 32-bit lane mask per bucket).
 template <int THREADS, int LAYOUT, int TILE = kTile>
 size_t scatter_smem_bytes(int buckets, bool bulk = false) {
   const size_t len = static_cast<size_t>(stage_len(TILE, buckets, bulk));
   const size_t stage = LAYOUT == EDPP_KO ? 4 * len : LAYOUT == EDPP_KVS_SOA ? 8 * len : TILE * 8;
   return stage + round_up(static_cast<size_t>(ScatterCfg<THREADS>::kWarps) * buckets * 2, 16) +
          2 * static_cast<size_t>(buckets) * 4 +
-         static_cast<size_t>(ScatterCfg<THREADS>::kWarps) * peer_table_bytes(buckets);
+         static_cast<size_t>(ScatterCfg<THREADS>::kWarps) * buckets * 4;
 }
 
 // Two blocks per SM (their staging fills shared memory): at most 64 registers.
-// kWide: more than 256 buckets, ranked through the leader table; up to 256
-// buckets the register counts and lane masks.  Two kernels rather than one
-// carrying every form: 16 / 32 / 64 / 256 buckets 19 / 14 / 12 / 7% faster
-// at 2^28 pairs, 512 and 1024 even (one process, both builds).  A third
-// kernel for the register counts alone spilled and made 2 buckets 4% slower.
+// For fewer than index_buckets() buckets.
 //
 // kFused: the whole split in one cooperative launch, for inputs whose tiles are
 // all resident together.  The tile's bucket counts come from its own ranking;
@@ -259,7 +248,7 @@ __device__ __forceinline__ bool fused_starts(const FusedArgs &f, int t, int tile
   return true;
 }
 
-template <int THREADS, int LAYOUT, bool kWide, int TILE = kTile, bool kFused = false>
+template <int THREADS, int LAYOUT, int TILE = kTile, bool kFused = false>
 __global__ void __launch_bounds__(THREADS, 2)
     split_scatter_kernel(const int32_t *__restrict__ keys_in, int32_t *__restrict__ keys_out,
                          const int32_t *__restrict__ vals_in, int32_t *__restrict__ vals_out,
@@ -269,7 +258,7 @@ __global__ void __launch_bounds__(THREADS, 2)
   using C = ScatterCfg<THREADS, TILE>;
   extern __shared__ __align__(128) unsigned char smem[];
   // Layout: stage (keys[L] + vals[L] with L = stage_len, or pairs[TILE]) |
-  // cnt16 | toff | gofs | peer tables.  `bulk` (KO / SOA only): runs go out by
+  // cnt16 | toff | gofs | lane masks.  `bulk` (KO / SOA only): runs go out by
   // bulk copies.
   const int slen = stage_len(TILE, buckets, bulk);
   int32_t *s_keys = reinterpret_cast<int32_t *>(smem);
@@ -281,7 +270,7 @@ __global__ void __launch_bounds__(THREADS, 2)
   int32_t *toff = reinterpret_cast<int32_t *>(
       smem + stage + round_up(static_cast<size_t>(C::kWarps) * buckets * 2, 16));
   int32_t *gofs = toff + buckets;
-  unsigned char *s_peer = reinterpret_cast<unsigned char *>(gofs + buckets);  // [kWarps][table]
+  uint32_t *s_peer = reinterpret_cast<uint32_t *>(gofs + buckets);  // [kWarps][buckets]
   __shared__ alignas(8) uint64_t bar;
 
   const int64_t t = blockIdx.x;
@@ -320,9 +309,8 @@ __global__ void __launch_bounds__(THREADS, 2)
     }
   }
   for (int i = tid; i < C::kWarps * buckets; i += THREADS) cnt16[i] = 0;
-  if (!kWide && buckets > (1 << kRegBits))  // the lane masks start empty
-    for (int i = tid; i < C::kWarps * buckets; i += THREADS)
-      reinterpret_cast<uint32_t *>(s_peer)[i] = 0u;
+  if (buckets > (1 << kRegBits))  // the lane masks start empty
+    for (int i = tid; i < C::kWarps * buckets; i += THREADS) s_peer[i] = 0u;
   // This thread's buckets for the per-bucket combine below; the first
   // kHisPre of their global run starts (his[b*T + t], one 32-byte sector
   // each) are loaded now, so the round trip overlaps the tile's ranking.
@@ -342,8 +330,7 @@ __global__ void __launch_bounds__(THREADS, 2)
   const unsigned lt = lanemask_lt();
   const int kbits = 31 - __clz(buckets);
   uint16_t *my_cnt = cnt16 + w * buckets;
-  uint32_t *my_or = reinterpret_cast<uint32_t *>(s_peer) + w * buckets;  // up to 8 bits
-  uint8_t *my_last = s_peer + w * 256;                                  // above 8 bits
+  uint32_t *my_or = s_peer + w * buckets;
   int32_t kk[C::kIters];
   int32_t vv[C::kIters];
   uint32_t rk[(C::kIters + 1) / 2];  // two 16-bit ranks per register
@@ -368,7 +355,7 @@ __global__ void __launch_bounds__(THREADS, 2)
     }
     const int b = valid ? static_cast<int>((static_cast<unsigned>(key) >> shift) & mask) : -1;
     const unsigned vmask = __ballot_sync(0xffffffffu, valid);
-    if (!kWide && kbits <= kRegBits) {
+    if (kbits <= kRegBits) {
       unsigned peers = vmask, mine = vmask;
       for (int i = 0; i < kbits; ++i) {
         const unsigned bb = __ballot_sync(0xffffffffu, (b >> i) & 1);
@@ -384,30 +371,17 @@ __global__ void __launch_bounds__(THREADS, 2)
       else rk[it >> 1] = r;
       continue;
     }
-    unsigned peers;
-    if (!kWide) {
-      // every lane ORs its bit into its bucket's mask: the mask read back is
-      // the lane's peer group (2^28 pairs against the leader table below,
-      // in one kernel with it: 32 / 64 / 256 buckets 6 / 5 / 2% faster)
-      if (valid) atomicOr(&my_or[b], 1u << lane);
-      __syncwarp();
-      peers = valid ? my_or[b] : 0u;
-    } else {
-      // the lanes sharing the low 8 bucket bits agree on one leader lane
-      // (whichever write lands), 5 votes on the leader's lane number find
-      // that group, and one vote per bucket bit above the 8th splits it
-      // (a lane-mask table of all buckets would halve the blocks per SM)
-      if (valid) my_last[b & 255] = static_cast<uint8_t>(lane);
-      __syncwarp();
-      peers = match_low_bits(valid ? my_last[b & 255] : 0u, 5, vmask);
-      peers &= match_low_bits(static_cast<unsigned>(b) >> 8, kbits - 8, vmask);
-    }
+    // every lane ORs its bit into its bucket's mask: the mask read back is the
+    // lane's peer group
+    if (valid) atomicOr(&my_or[b], 1u << lane);
+    __syncwarp();
+    const unsigned peers = valid ? my_or[b] : 0u;
     const unsigned lower = peers & lt;
     const uint16_t before = valid ? my_cnt[b] : 0;
     __syncwarp();
     if (valid && lower == 0u) {
       my_cnt[b] = static_cast<uint16_t>(before + __popc(peers));
-      if (!kWide) my_or[b] = 0u;  // the group's lowest lane empties the mask
+      my_or[b] = 0u;  // the group's lowest lane empties the mask
     }
     __syncwarp();
     kk[it] = key;
@@ -416,7 +390,7 @@ __global__ void __launch_bounds__(THREADS, 2)
     if (it & 1) rk[it >> 1] |= r << 16;
     else rk[it >> 1] = r;
   }
-  if (!kWide && kbits <= kRegBits && lane < buckets) my_cnt[lane] = static_cast<uint16_t>(lane_cnt);
+  if (kbits <= kRegBits && lane < buckets) my_cnt[lane] = static_cast<uint16_t>(lane_cnt);
   __syncthreads();
 
   // -- per bucket: tile count, tile offset, then each warp's first slot --
@@ -505,7 +479,7 @@ __global__ void __launch_bounds__(THREADS, 2)
   // stretches; write from registers, skipping the shared-memory re-layout
   // (2^28 pairs: 1.21 -> 1.11 ms; at 4 buckets even, at 8 and more slower,
   // the stores' sectors being only partly filled) --
-  if (!kWide && buckets <= kDirectBuckets) {
+  if (buckets <= kDirectBuckets) {
 #pragma unroll
     for (int it = 0; it < C::kIters; ++it) {
       const int pos = w * C::kSeg + it * 32 + lane;
@@ -543,7 +517,7 @@ __global__ void __launch_bounds__(THREADS, 2)
       }
     }
   }
-  if (!kWide && bulk) {
+  if (bulk) {
     // -- write out: per bucket run, plain stores for the ragged ends and one
     // bulk copy per array for the 16-byte-aligned middle --
     fence_proxy_async_smem();  // the re-layout's writes before the copies read them
@@ -597,6 +571,14 @@ __global__ void __launch_bounds__(THREADS, 2)
   }
 }
 
+}  // namespace
+}  // namespace edpp
+
+#include "split_index.cuh"
+
+namespace edpp {
+namespace {
+
 // bucket_start[b] = his[b*T] (gatherStartPos, split_kernel.cl:320-332).
 __global__ void bucket_start_kernel(const int32_t *his, int64_t tiles, int buckets,
                                     int32_t *start) {
@@ -608,83 +590,141 @@ size_t his_bytes(int64_t tiles, int buckets) {
   return round_up(static_cast<size_t>(tiles) * buckets * 4, 256);
 }
 
-template <int THREADS, int LAYOUT, bool kWide> int set_smem_attr() {
+// From this many buckets on the scatter stages positions (split_index.cuh).
+// Whole split of 2^28 elements, element staging against position staging (ms):
+// KVS_SOA 16 buckets 1.144 / 1.138, 32 1.232 / 1.116, 256 1.513 / 1.242;
+// KVS_AOS 8 buckets 1.370 / 1.326, 256 1.590 / 1.339; KO 32 buckets 0.974 /
+// 0.986, 64 1.009 / 0.989, 256 1.233 / 1.092.
+template <int LAYOUT> constexpr int index_buckets() {
+  return LAYOUT == EDPP_KO ? 64 : LAYOUT == EDPP_KVS_SOA ? 32 : 8;
+}
+
+// Dynamic shared-memory limit of `kernel` raised to `bytes`, once per device;
+// `resident` gets how many blocks with that much fit this device.
+template <auto kernel> int prepare_kernel(int threads, size_t bytes, int64_t *resident) {
   static std::once_flag once[64];
   static int status[64];
+  static int64_t fit[64];
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) dev = 0;
   std::call_once(once[dev], [&] {
-    const size_t bytes = scatter_smem_bytes<THREADS, LAYOUT>(kWide ? kOnePassMax : 256, true);
-    status[dev] = cuda_status(cudaFuncSetAttribute(split_scatter_kernel<THREADS, LAYOUT, kWide>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   static_cast<int>(bytes)));
+    int per_sm = 0;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(bytes));
+    if (e == cudaSuccess)
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, bytes);
+    status[dev] = cuda_status(e);
+    fit[dev] = static_cast<int64_t>(per_sm) * device_sm_count();
   });
+  if (resident) *resident = fit[dev];
   return status[dev];
 }
 
-template <int THREADS, int LAYOUT>
-int launch_scatter(const int32_t *keys_in, int32_t *keys_out, const int32_t *vals_in,
-                   int32_t *vals_out, int64_t n, int buckets, int shift, int64_t tiles,
-                   const int32_t *his, bool tma, cudaStream_t st) {
-  const bool wide = buckets > 256;
-  const int s = wide ? set_smem_attr<THREADS, LAYOUT, true>() : set_smem_attr<THREADS, LAYOUT, false>();
-  if (s != EDPP_OK) return s;
-  const bool bulk = LAYOUT != EDPP_KVS_AOS && buckets > kDirectBuckets &&
-                    buckets <= kBulkBuckets && aligned16(keys_out) &&
-                    (LAYOUT != EDPP_KVS_SOA || aligned16(vals_out));
-  const size_t smem = scatter_smem_bytes<THREADS, LAYOUT>(buckets, bulk);
+// How many blocks of `kernel` with `bytes` of shared memory fit this device.
+template <auto kernel> int blocks_that_fit(int threads, size_t bytes, int64_t *resident) {
+  static std::once_flag once[64];
+  static int status[64];
+  static int64_t fit[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) dev = 0;
+  std::call_once(once[dev], [&] {
+    int per_sm = 0;
+    status[dev] = cuda_status(
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, bytes));
+    fit[dev] = static_cast<int64_t>(per_sm) * device_sm_count();
+  });
+  *resident = fit[dev];
+  return status[dev];
+}
+
+constexpr int kScatterThreads = 512;
+
+// A split's arrays and shape, and how it is to run.
+struct SplitArgs {
+  const int32_t *keys_in;
+  int32_t *keys_out;
+  const int32_t *vals_in;
+  int32_t *vals_out;
+  int32_t *bucket_start;
+  int64_t n;
+  int buckets, shift;
+  bool tma;    // inputs 16-byte aligned
+  bool exact;  // rank by peer groups (position staging only)
+};
+
+template <int LAYOUT> bool bulk_runs(const SplitArgs &a) {
+  return LAYOUT != EDPP_KVS_AOS && a.buckets > kDirectBuckets && a.buckets <= kBulkBuckets &&
+         aligned16(a.keys_out) && (LAYOUT != EDPP_KVS_SOA || aligned16(a.vals_out));
+}
+
+template <int LAYOUT>
+int launch_scatter(const SplitArgs &a, int64_t tiles, const int32_t *his, cudaStream_t st) {
   const unsigned grid = static_cast<unsigned>(tiles);
-  if (wide)
-    split_scatter_kernel<THREADS, LAYOUT, true><<<grid, THREADS, smem, st>>>(
-        keys_in, keys_out, vals_in, vals_out, n, buckets, shift, tiles, his, tma, bulk,
-        kDefaultWaitNs, fault_word(), FusedArgs{});
-  else
-    split_scatter_kernel<THREADS, LAYOUT, false><<<grid, THREADS, smem, st>>>(
-        keys_in, keys_out, vals_in, vals_out, n, buckets, shift, tiles, his, tma, bulk,
-        kDefaultWaitNs, fault_word(), FusedArgs{});
+  if (a.buckets >= index_buckets<LAYOUT>()) {
+    constexpr auto kernel = split_index_kernel<LAYOUT, kTile, false>;
+    const int s = prepare_kernel<kernel>(
+        kIndexThreads, index_smem_bytes<LAYOUT, kTile>(kOnePassMax), nullptr);
+    if (s != EDPP_OK) return s;
+    kernel<<<grid, kIndexThreads, index_smem_bytes<LAYOUT, kTile>(a.buckets), st>>>(
+        a.keys_in, a.keys_out, a.vals_in, a.vals_out, a.n, a.buckets, a.shift, tiles, his, a.tma,
+        a.exact, kDefaultWaitNs, fault_word(), FusedArgs{});
+    return launch_status();
+  }
+  constexpr auto kernel = split_scatter_kernel<kScatterThreads, LAYOUT, kTile, false>;
+  const int s = prepare_kernel<kernel>(
+      kScatterThreads, scatter_smem_bytes<kScatterThreads, LAYOUT, kTile>(index_buckets<LAYOUT>(), true),
+      nullptr);
+  if (s != EDPP_OK) return s;
+  const bool bulk = bulk_runs<LAYOUT>(a);
+  kernel<<<grid, kScatterThreads, scatter_smem_bytes<kScatterThreads, LAYOUT, kTile>(a.buckets, bulk),
+           st>>>(a.keys_in, a.keys_out, a.vals_in, a.vals_out, a.n, a.buckets, a.shift, tiles, his,
+                 a.tma, bulk, kDefaultWaitNs, fault_word(), FusedArgs{});
   return launch_status();
 }
 
 // The fused split with tiles of TILE elements; EDPP_ENOMEM (nothing launched)
 // when the tiles cannot all be resident or the cooperative launch is refused.
-template <int LAYOUT, bool kWide, int TILE>
-int launch_fused(const int32_t *keys_in, int32_t *keys_out, const int32_t *vals_in,
-                 int32_t *vals_out, int32_t *bucket_start, int64_t n, int buckets, int shift,
-                 char *ws, bool tma, cudaStream_t st) {
-  constexpr int THREADS = 512;
-  auto *kernel = split_scatter_kernel<THREADS, LAYOUT, kWide, TILE, true>;
-  static std::once_flag once[64];
-  static int resident[64];  // of the largest bucket count
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) dev = 0;
-  std::call_once(once[dev], [dev, kernel] {
-    const size_t bytes = scatter_smem_bytes<THREADS, LAYOUT, TILE>(kWide ? kOnePassMax : 256, true);
-    int per_sm = 0;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(bytes)) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, THREADS, bytes) !=
-            cudaSuccess) {
-      per_sm = 0;
-      cudaGetLastError();
-    }
-    resident[dev] = per_sm * device_sm_count();
-  });
-  int64_t tiles = (n + TILE - 1) / TILE;
-  if (tiles > resident[dev]) return EDPP_ENOMEM;
-  bool bulk = LAYOUT != EDPP_KVS_AOS && buckets > kDirectBuckets && buckets <= kBulkBuckets &&
-              aligned16(keys_out) && (LAYOUT != EDPP_KVS_SOA || aligned16(vals_out));
-  const size_t smem = scatter_smem_bytes<THREADS, LAYOUT, TILE>(buckets, bulk);
+template <int LAYOUT, int TILE>
+int launch_fused(const SplitArgs &a, char *ws, cudaStream_t st) {
+  constexpr auto index = split_index_kernel<LAYOUT, TILE, true>;
+  constexpr auto scatter = split_scatter_kernel<kScatterThreads, LAYOUT, TILE, true>;
+  const bool by_index = a.buckets >= index_buckets<LAYOUT>();
+  int64_t resident = 0;
+  int s;
+  if (!by_index) {
+    s = prepare_kernel<scatter>(
+        kScatterThreads, scatter_smem_bytes<kScatterThreads, LAYOUT, TILE>(index_buckets<LAYOUT>(), true),
+        &resident);
+  } else if (a.buckets > 256) {
+    s = prepare_kernel<index>(kIndexThreads, index_smem_bytes<LAYOUT, TILE>(kOnePassMax),
+                                    &resident);
+  } else {
+    // the limit stays at the larger count's
+    s = prepare_kernel<index>(kIndexThreads, index_smem_bytes<LAYOUT, TILE>(kOnePassMax),
+                                    nullptr);
+    if (s == EDPP_OK) s = blocks_that_fit<index>(kIndexThreads, index_smem_bytes<LAYOUT, TILE>(256), &resident);
+  }
+  int64_t tiles = (a.n + TILE - 1) / TILE;
+  if (s != EDPP_OK || tiles > resident) return EDPP_ENOMEM;
   if (cudaMemsetAsync(ws, 0, 16, st) != cudaSuccess) return EDPP_ECUDA;
-  int32_t *his = reinterpret_cast<int32_t *>(ws + 256);
-  FusedArgs fused{reinterpret_cast<unsigned *>(ws), his, bucket_start};
+  SplitArgs v = a;
+  const int32_t *his = nullptr;
+  FusedArgs fused{reinterpret_cast<unsigned *>(ws), reinterpret_cast<int32_t *>(ws + 256),
+                  a.bucket_start};
+  bool flag = by_index ? a.exact : bulk_runs<LAYOUT>(a);
   uint64_t timeout_ns = kDefaultWaitNs;
   unsigned *fault = fault_word();
-  void *args[] = {&keys_in, &keys_out, &vals_in, &vals_out, &n,    &buckets,    &shift, &tiles,
-                  &his,     &tma,      &bulk,    &timeout_ns, &fault, &fused};
-  if (cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(kernel),
-                                  dim3(static_cast<unsigned>(tiles)), dim3(THREADS), args, smem,
+  void *args[] = {&v.keys_in, &v.keys_out, &v.vals_in, &v.vals_out, &v.n,   &v.buckets, &v.shift,
+                  &tiles,     &his,        &v.tma,     &flag,       &timeout_ns, &fault, &fused};
+  const size_t smem = by_index
+                          ? index_smem_bytes<LAYOUT, TILE>(a.buckets)
+                          : scatter_smem_bytes<kScatterThreads, LAYOUT, TILE>(a.buckets, flag);
+  if (cudaLaunchCooperativeKernel(by_index ? reinterpret_cast<const void *>(index)
+                                           : reinterpret_cast<const void *>(scatter),
+                                  dim3(static_cast<unsigned>(tiles)),
+                                  dim3(by_index ? kIndexThreads : kScatterThreads), args, smem,
                                   st) != cudaSuccess) {
     cudaGetLastError();
     return EDPP_ENOMEM;
@@ -709,41 +749,31 @@ size_t fused_ws_bytes(int64_t n, int buckets) {
   return 256 + 4 * static_cast<size_t>(min64(kFusedWords, (n + kSmallTile - 1) / kSmallTile * buckets));
 }
 
-template <int LAYOUT, bool kWide>
-int split_fused(const int32_t *keys_in, int32_t *keys_out, const int32_t *vals_in,
-                int32_t *vals_out, int32_t *bucket_start, int64_t n, int buckets, int shift,
-                char *ws, bool tma, cudaStream_t st) {
+template <int LAYOUT> int split_fused(const SplitArgs &a, char *ws, cudaStream_t st) {
   const int64_t sms = device_sm_count();
   auto fits = [&](int64_t tile, int64_t blocks) {
-    const int64_t tiles = (n + tile - 1) / tile;
-    return tiles <= blocks && tiles * buckets <= kFusedWords;
+    const int64_t tiles = (a.n + tile - 1) / tile;
+    return tiles <= blocks && tiles * a.buckets <= kFusedWords;
   };
-  if (fits(kSmallTile, sms))
-    return launch_fused<LAYOUT, kWide, kSmallTile>(keys_in, keys_out, vals_in, vals_out,
-                                                   bucket_start, n, buckets, shift, ws, tma, st);
-  if (fits(kMidTile, sms))
-    return launch_fused<LAYOUT, kWide, kMidTile>(keys_in, keys_out, vals_in, vals_out,
-                                                 bucket_start, n, buckets, shift, ws, tma, st);
-  if (fits(kTile, 2 * sms))
-    return launch_fused<LAYOUT, kWide, kTile>(keys_in, keys_out, vals_in, vals_out, bucket_start,
-                                              n, buckets, shift, ws, tma, st);
+  if (fits(kSmallTile, sms)) return launch_fused<LAYOUT, kSmallTile>(a, ws, st);
+  if (fits(kMidTile, sms)) return launch_fused<LAYOUT, kMidTile>(a, ws, st);
+  if (fits(kTile, 2 * sms)) return launch_fused<LAYOUT, kTile>(a, ws, st);
   return EDPP_ENOMEM;
 }
 
 template <int LAYOUT>
 int split_layout(const int32_t *keys_in, int32_t *keys_out, int32_t *bucket_start, int64_t n,
                  int buckets, const int32_t *vals_in, int32_t *vals_out, void *ws, size_t ws_bytes,
-                 cudaStream_t st, int shift = 0) {
+                 cudaStream_t st, int shift = 0, bool exact = false) {
   if (buckets > kOnePassMax) return EDPP_EINVAL;  // callers take two passes from 2048 on
   const int64_t tiles = (n + kTile - 1) / kTile;
   int32_t *his = static_cast<int32_t *>(ws);
   const int64_t hlen = tiles * buckets;
   void *scan_ws = static_cast<char *>(ws) + his_bytes(tiles, buckets);
   const size_t scan_ws_bytes = ws_bytes - his_bytes(tiles, buckets);
-  bool tma = aligned16(keys_in) && (LAYOUT != EDPP_KVS_SOA || aligned16(vals_in));
-  int s = (buckets > 256 ? split_fused<LAYOUT, true> : split_fused<LAYOUT, false>)(
-      keys_in, keys_out, vals_in, vals_out, bucket_start, n, buckets, shift,
-      static_cast<char *>(ws), tma, st);
+  const SplitArgs a{keys_in, keys_out, vals_in, vals_out, bucket_start, n, buckets, shift,
+                    aligned16(keys_in) && (LAYOUT != EDPP_KVS_SOA || aligned16(vals_in)), exact};
+  int s = split_fused<LAYOUT>(a, static_cast<char *>(ws), st);
   if (s != EDPP_ENOMEM) return s;
   split_hist_kernel<LAYOUT><<<static_cast<unsigned>(tiles), kHistThreads, 0, st>>>(
       keys_in, n, buckets, shift, tiles, his, aligned16(keys_in));
@@ -756,8 +786,7 @@ int split_layout(const int32_t *keys_in, int32_t *keys_out, int32_t *bucket_star
     s = launch_status();
     if (s != EDPP_OK) return s;
   }
-  return launch_scatter<512, LAYOUT>(keys_in, keys_out, vals_in, vals_out, n, buckets, shift,
-                                     tiles, his, tma, st);
+  return launch_scatter<LAYOUT>(a, tiles, his, st);
 }
 
 // From kLsdBuckets buckets on, a split is two stable passes through a
@@ -921,6 +950,23 @@ int edpp_split_i32(const int32_t *keys_in, int32_t *keys_out, int32_t *bucket_st
 }
 
 }  // extern "C"
+
+extern "C" int edpp_selftest_split_exact(const int32_t *keys_in, int32_t *keys_out,
+                                         int32_t *bucket_start, int64_t length, int buckets,
+                                         int layout, const int32_t *vals_in, int32_t *vals_out,
+                                         void *ws, size_t ws_bytes, void *stream) {
+  using namespace edpp;
+  if (length <= 0 || length > INT32_MAX || !keys_in || !keys_out) return EDPP_EINVAL;
+  if (buckets < 1 || buckets > kOnePassMax || (buckets & (buckets - 1))) return EDPP_EINVAL;
+  if (layout != EDPP_KO && layout != EDPP_KVS_AOS && layout != EDPP_KVS_SOA) return EDPP_EINVAL;
+  if (layout == EDPP_KVS_SOA && (!vals_in || !vals_out)) return EDPP_EINVAL;
+  if (!ws || ws_bytes < split_ws_bytes(length, buckets)) return EDPP_ENOMEM;
+  const auto run = layout == EDPP_KO ? split_layout<EDPP_KO>
+                   : layout == EDPP_KVS_SOA ? split_layout<EDPP_KVS_SOA>
+                                            : split_layout<EDPP_KVS_AOS>;
+  return run(keys_in, keys_out, bucket_start, length, buckets, vals_in, vals_out, ws, ws_bytes,
+             as_stream(stream), 0, /*exact=*/true);
+}
 
 // ---- LSD radix sort on the stable split -----------------------------------------
 // Sorts (key, value) pairs by the key's bit pattern (unsigned order) over bits

@@ -1,0 +1,249 @@
+// split_index.cuh — split scatter that stages source positions (split.cu).
+//
+// A tile stays in shared memory as loaded.  Ranking takes one shared-memory
+// atomic per element: the old value of the (warp, bucket) counter is the
+// element's rank among its warp's elements of the bucket.  What is re-laid out
+// in bucket order is only the 16-bit source position; the write-out fetches key
+// and value from there.
+//
+// Atomics of one warp instruction on one counter, and of successive
+// instructions, have returned in lane and program order wherever it was
+// looked at, but nothing promises that, so the write-out checks it: positions
+// must ascend within every bucket's run.  A tile that fails is ranked again by
+// peer groups (exact, slow) and written over.
+//
+// Bound by the shared-memory pipe: 27 wavefronts per 32 pairs at 256 buckets
+// (the returning atomic 8, the random reads of key and value 7, the position
+// store and the slot lookup 3 each) against 34 for per-warp lane masks with
+// the pairs themselves re-laid out, and nothing in the ranking waits for the
+// step before.  Scatter alone, 2^28 pairs, 256 buckets: 1.30 -> 1.03 ms; whole
+// splits at index_buckets() in split.cu.  512 and 1024 buckets ranked by a
+// leader table before: 1.85 -> 1.51 and 2.57 -> 2.21 ms.
+#pragma once
+
+namespace edpp {
+namespace {
+
+constexpr int kIndexThreads = 512;
+template <int TILE> struct IndexCfg {
+  static constexpr int kWarps = kIndexThreads / 32;
+  static constexpr int kSeg = TILE / kWarps;
+  static constexpr int kIters = kSeg / 32;
+};
+
+// tile | positions | counters of 16 bits per (warp, bucket) | totals | run starts
+template <int LAYOUT, int TILE> size_t index_smem_bytes(int buckets) {
+  return static_cast<size_t>(TILE) * (LAYOUT == EDPP_KO ? 4 : 8) + 2 * static_cast<size_t>(TILE) +
+         round_up(static_cast<size_t>(IndexCfg<TILE>::kWarps) * buckets * 2, 16) +
+         8 * static_cast<size_t>(buckets);
+}
+
+template <int LAYOUT, int TILE, bool kFused>
+__global__ void __launch_bounds__(kIndexThreads, 2)
+    split_index_kernel(const int32_t *__restrict__ keys_in, int32_t *__restrict__ keys_out,
+                       const int32_t *__restrict__ vals_in, int32_t *__restrict__ vals_out,
+                       int64_t n, int buckets, int shift, int64_t tiles,
+                       const int32_t *__restrict__ his, bool tma, bool exact, uint64_t timeout_ns,
+                       unsigned *fault, FusedArgs fused) {
+  using C = IndexCfg<TILE>;
+  constexpr int THREADS = kIndexThreads;
+  extern __shared__ __align__(128) unsigned char smem[];
+  int32_t *s_keys = reinterpret_cast<int32_t *>(smem);
+  int32_t *s_vals = s_keys + TILE;                 // SOA only
+  int2 *s_pairs = reinterpret_cast<int2 *>(smem);  // AOS only
+  uint16_t *s_pos = reinterpret_cast<uint16_t *>(smem + TILE * (LAYOUT == EDPP_KO ? 4 : 8));
+  uint16_t *cnt16 = s_pos + TILE;
+  int32_t *toff = reinterpret_cast<int32_t *>(
+      reinterpret_cast<unsigned char *>(cnt16) + round_up(static_cast<size_t>(C::kWarps) * buckets * 2, 16));
+  int32_t *gofs = toff + buckets;
+  __shared__ alignas(8) uint64_t bar;
+  __shared__ int32_t s_wsum[32];
+
+  const int64_t t = blockIdx.x;
+  const int64_t base = t * TILE;
+  const int count = static_cast<int>(min64(TILE, n - base));
+  const unsigned mask = static_cast<unsigned>(buckets - 1);
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+
+  // -- load the tile (bulk copies for the 16-byte-aligned prefix) --
+  if (tid == 0) {
+    mbar_init(&bar, 1);
+    fence_mbar_init();
+  }
+  __syncthreads();
+  uint32_t bulk_elems = 0;
+  if (tma) bulk_elems = (LAYOUT == EDPP_KVS_AOS) ? (count & ~1) : (count & ~3);
+  if (tid == 0 && bulk_elems) {
+    mbar_arrive_expect_tx(&bar, bulk_elems * (LAYOUT == EDPP_KO ? 4 : 8));
+    if (LAYOUT == EDPP_KVS_AOS) {
+      tma_load_1d(s_pairs, keys_in + 2 * base, bulk_elems * 8, &bar);
+    } else {
+      tma_load_1d(s_keys, keys_in + base, bulk_elems * 4, &bar);
+      if (LAYOUT == EDPP_KVS_SOA) tma_load_1d(s_vals, vals_in + base, bulk_elems * 4, &bar);
+    }
+  }
+  for (int i = static_cast<int>(bulk_elems) + tid; i < count; i += THREADS) {
+    if (LAYOUT == EDPP_KVS_AOS) {
+      s_pairs[i] = make_int2(keys_in[2 * (base + i)], keys_in[2 * (base + i) + 1]);
+    } else {
+      s_keys[i] = keys_in[base + i];
+      if (LAYOUT == EDPP_KVS_SOA) s_vals[i] = vals_in[base + i];
+    }
+  }
+  uint32_t *cnt_words = reinterpret_cast<uint32_t *>(cnt16);  // two counters per word
+  const int row = buckets / 2;                                // words per warp
+  for (int i = tid; i < C::kWarps * row; i += THREADS) cnt_words[i] = 0u;
+  const int per = (buckets + THREADS - 1) / THREADS;
+  const int b_lo = min(buckets, tid * per), b_hi = min(buckets, b_lo + per);
+  constexpr int kHisPre = 2;  // 512 threads serve up to 1024 buckets
+  int32_t his_pre[kHisPre];
+#pragma unroll
+  for (int k = 0; k < kHisPre; ++k)
+    his_pre[k] = !kFused && b_lo + k < b_hi
+                     ? __ldg(his + static_cast<int64_t>(b_lo + k) * tiles + t) : 0;
+  if (bulk_elems) {
+    if (!mbar_wait_bounded(&bar, 0, timeout_ns, fault)) return;
+  }
+  __syncthreads();
+  auto key_of = [&](int pos) { return LAYOUT == EDPP_KVS_AOS ? s_pairs[pos].x : s_keys[pos]; };
+  auto bucket_of = [&](int32_t key) {
+    return static_cast<int>((static_cast<unsigned>(key) >> shift) & mask);
+  };
+
+  // -- rank: warp w owns tile positions [w*kSeg, (w+1)*kSeg), in order --
+  uint32_t br[C::kIters];  // bucket | rank << 16
+  uint32_t *my_words = cnt_words + w * row;
+#pragma unroll
+  for (int it = 0; it < C::kIters; ++it) {
+    const int pos = w * C::kSeg + it * 32 + lane;
+    br[it] = pos < count ? static_cast<uint32_t>(bucket_of(key_of(pos))) : 0u;
+  }
+#pragma unroll
+  for (int it = 0; it < C::kIters; ++it) {
+    const int pos = w * C::kSeg + it * 32 + lane;
+    const uint32_t sh = (br[it] & 1u) * 16u;
+    if (pos < count)
+      br[it] |= ((atomicAdd(&my_words[br[it] >> 1], 1u << sh) >> sh) & 0xffffu) << 16;
+  }
+  __syncthreads();
+
+  // -- per bucket: tile count, tile offset, then each warp's first slot
+  // (cnt16[w][b] becomes the tile slot of warp w's first element of bucket b) --
+  int32_t my_total = 0;
+  for (int b = b_lo; b < b_hi; ++b) {
+    int32_t tot = 0;
+#pragma unroll 8
+    for (int ww = 0; ww < C::kWarps; ++ww) tot += cnt16[ww * buckets + b];
+    toff[b] = tot;
+    my_total += tot;
+  }
+  int32_t incl = my_total;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int32_t y = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += y;
+  }
+  if (lane == 31) s_wsum[w] = incl;
+  __syncthreads();
+  int32_t run = incl - my_total;
+#pragma unroll
+  for (int k = 0; k < C::kWarps; ++k)
+    if (k < w) run += s_wsum[k];
+  if (kFused) {
+    // the position area is free until the re-layout
+    if (!fused_starts<THREADS>(fused, static_cast<int>(t), static_cast<int>(tiles), buckets, toff,
+                               gofs, reinterpret_cast<int32_t *>(s_pos), timeout_ns, fault))
+      return;
+#pragma unroll
+    for (int k = 0; k < kHisPre; ++k) his_pre[k] = b_lo + k < b_hi ? gofs[b_lo + k] : 0;
+  }
+#pragma unroll
+  for (int k = 0; k < kHisPre; ++k) {
+    const int b = b_lo + k;
+    if (b < b_hi) {
+      gofs[b] = his_pre[k] - run;  // output index of a slot of this run, minus the slot
+#pragma unroll 8
+      for (int ww = 0; ww < C::kWarps; ++ww) {
+        const int32_t c = cnt16[ww * buckets + b];
+        cnt16[ww * buckets + b] = static_cast<uint16_t>(run);
+        run += c;
+      }
+    }
+  }
+  __syncthreads();
+
+  // -- positions in bucket order --
+  if (!exact) {
+#pragma unroll
+    for (int it = 0; it < C::kIters; ++it) {
+      const int pos = w * C::kSeg + it * 32 + lane;
+      if (pos < count)
+        s_pos[cnt16[w * buckets + (br[it] & 0xffffu)] + (br[it] >> 16)] = static_cast<uint16_t>(pos);
+    }
+    __syncthreads();
+  }
+
+  // -- write out: consecutive threads write consecutive slots of a bucket run --
+  auto write_out = [&]() {
+    bool bad = false;
+#pragma unroll 4
+    for (int s0 = 0; s0 < TILE; s0 += THREADS) {
+      const int s = s0 + tid;
+      const bool valid = s < count;
+      const int pos = valid ? s_pos[s] : 0;
+      int32_t key = 0, val = 0;
+      if (LAYOUT == EDPP_KVS_AOS) {
+        const int2 p = s_pairs[pos];
+        key = p.x;
+        val = p.y;
+      } else {
+        key = s_keys[pos];
+        if (LAYOUT == EDPP_KVS_SOA) val = s_vals[pos];
+      }
+      const int b = bucket_of(key);
+      // (bucket, position) ascends from slot to slot
+      const int mine = b * TILE + pos;
+      int before = __shfl_up_sync(0xffffffffu, mine, 1);
+      if (lane == 0 && valid) {
+        const int q = s > 0 ? s_pos[s - 1] : 0;
+        before = s > 0 ? bucket_of(key_of(q)) * TILE + q : -1;
+      }
+      bad |= valid && before >= mine;
+      if (valid) {
+        const int64_t o = static_cast<int64_t>(gofs[b]) + s;
+        if (LAYOUT == EDPP_KVS_AOS) {
+          reinterpret_cast<int2 *>(keys_out)[o] = make_int2(key, val);
+        } else {
+          keys_out[o] = key;
+          if (LAYOUT == EDPP_KVS_SOA) vals_out[o] = val;
+        }
+      }
+    }
+    return bad;
+  };
+  bool bad = exact;
+  if (!exact) bad = write_out();
+  if (__syncthreads_or(bad)) {
+    // exact ranks: the lanes of a bucket count their lower peers, warp by warp
+    // in input order, advancing the warp's slot of the bucket
+    const unsigned lt = lanemask_lt();
+    for (int it = 0; it < C::kIters; ++it) {
+      const int pos = w * C::kSeg + it * 32 + lane;
+      const bool valid = pos < count;
+      const int b = valid ? bucket_of(key_of(pos)) : 0;
+      const unsigned vmask = __ballot_sync(0xffffffffu, valid);
+      const unsigned peers = match_low_bits(static_cast<unsigned>(b), 31 - __clz(buckets), vmask);
+      const int before = valid ? cnt16[w * buckets + b] : 0;
+      __syncwarp();
+      if (valid && (peers & lt) == 0u)
+        cnt16[w * buckets + b] = static_cast<uint16_t>(before + __popc(peers));
+      __syncwarp();
+      if (valid) s_pos[before + __popc(peers & lt)] = static_cast<uint16_t>(pos);
+    }
+    __syncthreads();
+    write_out();
+  }
+}
+
+}  // namespace
+}  // namespace edpp

@@ -538,6 +538,15 @@ int edpp_autotune_plain(int primitive, const void *in, void *out, const int32_t 
                         void *stream, int reps, void *flush, size_t flush_bytes,
                         int *best_variant, float *best_ms, float *variant_ms);
 
+/* ---- split ranking self-test --------------------------------------------- */
+
+/* edpp_split_i32 for up to 1024 buckets with the tiles ranked the way a tile
+ * is whose quick ranking failed its check (position-staged tiles only; the
+ * others run as usual).  Same arguments and results. */
+int edpp_selftest_split_exact(const int32_t *keys_in, int32_t *keys_out, int32_t *bucket_start,
+                              int64_t length, int buckets, int layout, const int32_t *vals_in,
+                              int32_t *vals_out, void *ws, size_t ws_bytes, void *stream);
+
 /* ---- bounded-wait self-test --------------------------------------------- */
 
 /* Runs a look-back scan over `length` int32 elements whose first tile is
