@@ -158,9 +158,15 @@ def check(status: int, what: str = "") -> None:
 
 # ---------------------------------------------------------------------------
 # device helpers
+_torch_module = None
+
+
 def _torch():
-    import torch  # imported lazily: the generators and the ABI load need no torch
-    return torch
+    global _torch_module
+    if _torch_module is None:
+        import torch  # imported lazily: the generators and the ABI load need no torch
+        _torch_module = torch
+    return _torch_module
 
 
 def _cuda_tensor(t, dtype=None, name="tensor"):
@@ -174,12 +180,35 @@ def _cuda_tensor(t, dtype=None, name="tensor"):
     return t
 
 
-def _p(t) -> ctypes.c_void_p:
-    return ctypes.c_void_p(t.data_ptr() if t is not None else 0)
+def _p(t) -> int | None:
+    """Device address of a tensor as ctypes takes it for a pointer argument."""
+    return t.data_ptr() if t is not None else None
+
+
+_raw_stream = None
+
+
+def _raw_stream_getter():
+    """() -> the current stream's handle on the current device.  The call path of a small
+    primitive is host time, and building a torch.cuda.Stream object per call cost 2 of its
+    10 us; torch's raw-handle query is used where this torch has it."""
+    global _raw_stream
+    torch = _torch()
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    if raw is not None:
+        device = torch.cuda.current_device
+        _raw_stream = lambda: raw(device())  # noqa: E731
+    else:
+        _raw_stream = lambda: torch.cuda.current_stream().cuda_stream  # noqa: E731
+    return _raw_stream
+
+
+def _stream() -> int:
+    return (_raw_stream or _raw_stream_getter())()
 
 
 def current_stream_handle() -> ctypes.c_void_p:
-    return ctypes.c_void_p(_torch().cuda.current_stream().cuda_stream)
+    return ctypes.c_void_p(_stream())
 
 
 def workspace(nbytes: int, device=None):
@@ -203,7 +232,7 @@ def _gs(kind, inp, loc, passes, out, method, ws):
         raise ValueError("inp shorter than loc")
     if out is None:
         out = torch.zeros(n, dtype=torch.int32, device=loc.device)
-    st = current_stream_handle()
+    st = _stream()
     if method == "auto":  # the faster schedule for this size
         direct = (lib().edpp_gather_prefers_direct if kind == "gather"
                   else lib().edpp_scatter_prefers_direct)
@@ -213,9 +242,8 @@ def _gs(kind, inp, loc, passes, out, method, ws):
         f = lib().edpp_gather_i32 if kind == "gather" else lib().edpp_scatter_i32
         check(f(_p(inp), _p(out), n, _p(loc), int(passes), st), kind)
     elif method in ("partition", "tiled"):
-        need = gs_workspace_bytes(kind, n, passes, method)
         if ws is None:
-            ws = workspace(need, loc.device)
+            ws = workspace(gs_workspace_bytes(kind, n, passes, method), loc.device)
         if method == "partition":
             f = lib().edpp_gather_i32_ws if kind == "gather" else lib().edpp_scatter_i32_ws
         else:
@@ -297,11 +325,18 @@ def scatter(inp, loc, passes: int = 1, out=None, method: str = "sweep", ws=None)
     return _gs("scatter", inp, loc, passes, out, method, ws)
 
 
-_SCAN_FN = {
-    ("int32", False): "edpp_scan_exclusive_i32", ("int32", True): "edpp_scan_inclusive_i32",
-    ("int64", False): "edpp_scan_exclusive_i64", ("int64", True): "edpp_scan_inclusive_i64",
-    ("float32", False): "edpp_scan_exclusive_f32", ("float32", True): "edpp_scan_inclusive_f32",
-}
+_SCAN_SUFFIX = {"int32": "i32", "int64": "i64", "float32": "f32"}
+_scan_table = {}  # torch dtype -> (dtype name, exclusive function, inclusive function)
+
+
+def _scan_entry(dtype):
+    torch = _torch()
+    for name, suffix in _SCAN_SUFFIX.items():
+        _scan_table[getattr(torch, name)] = (name, getattr(lib(), f"edpp_scan_exclusive_{suffix}"),
+                                             getattr(lib(), f"edpp_scan_inclusive_{suffix}"))
+    if dtype not in _scan_table:
+        raise TypeError(f"scan supports int32, int64, float32, got {dtype}")
+    return _scan_table[dtype]
 
 
 def scan_workspace_bytes(n: int, dtype: str, algo: str = "lookback") -> int:
@@ -311,18 +346,14 @@ def scan_workspace_bytes(n: int, dtype: str, algo: str = "lookback") -> int:
 def scan(x, inclusive: bool = False, algo: str = "lookback", out=None, ws=None):
     torch = _torch()
     _cuda_tensor(x, None, "x")
-    dt = str(x.dtype).replace("torch.", "")
-    if dt not in DTYPES:
-        raise TypeError(f"scan supports int32, int64, float32, got {x.dtype}")
+    dt, exclusive_fn, inclusive_fn = _scan_table.get(x.dtype) or _scan_entry(x.dtype)
     n = x.numel()
     if out is None:
         out = torch.empty_like(x)
-    need = scan_workspace_bytes(n, dt, algo)
     if ws is None:
-        ws = workspace(need, x.device)
-    fn = getattr(lib(), _SCAN_FN[(dt, bool(inclusive))])
-    check(fn(_p(x), _p(out), n, SCAN_ALGOS[algo], _p(ws), ws.numel(), current_stream_handle()),
-          "scan")
+        ws = workspace(scan_workspace_bytes(n, dt, algo), x.device)
+    check((inclusive_fn if inclusive else exclusive_fn)(_p(x), _p(out), n, SCAN_ALGOS[algo], _p(ws),
+                                                        ws.numel(), _stream()), "scan")
     return out
 
 
@@ -354,13 +385,12 @@ def split(keys, buckets: int, values=None, layout: str | None = None, bucket_sta
     if layout == "soa" and values_out is None:
         values_out = torch.empty_like(values)
     start = torch.empty(buckets, dtype=torch.int32, device=keys.device) if bucket_start else None
-    need = split_workspace_bytes(n, buckets, layout)
     if ws is None:
-        ws = workspace(need, keys.device)
+        ws = workspace(split_workspace_bytes(n, buckets, layout), keys.device)
     check(lib().edpp_split_i32(_p(keys), _p(keys_out), _p(start), n, int(buckets),
                                LAYOUTS[layout], _p(values if layout == "soa" else None),
                                _p(values_out if layout == "soa" else None), _p(ws), ws.numel(),
-                               current_stream_handle()), "split")
+                               _stream()), "split")
     return keys_out, (values_out if layout == "soa" else None), start
 
 
@@ -399,7 +429,7 @@ def radix_sort(keys, values=None, begin_bit=0, end_bit=32, keys_out=None, values
                        keys.device)
     check(lib().edpp_radix_sort_i32(_p(keys), _p(keys_out), _p(values), _p(values_out), n,
                                     int(begin_bit), int(end_bit), _p(ws), ws.numel(),
-                                    current_stream_handle()), "radix_sort")
+                                    _stream()), "radix_sort")
     return keys_out, values_out
 
 
@@ -413,7 +443,7 @@ def hash_join_count(r_keys, s_keys, buckets: int = 0, ws=None, partitioned: bool
     _cuda_tensor(r_keys, torch.int32, "r_keys")
     _cuda_tensor(s_keys, torch.int32, "s_keys")
     cnt = count if count is not None else torch.zeros(1, dtype=torch.int64, device=r_keys.device)
-    st = current_stream_handle()
+    st = _stream()
     if partitioned:
         if ws is None:
             ws = workspace(lib().edpp_hash_join_workspace_size(r_keys.numel(), s_keys.numel(),
@@ -495,7 +525,7 @@ def stream(op: str, a, b=None, scalar=3, out=None):
     n = a.numel()
     f = getattr(lib(), f"edpp_stream_{op}_{suffix}")
     s = float(scalar) if suffix == "f32" else int(scalar)
-    st = current_stream_handle()
+    st = _stream()
     if op == "copy":
         r = f(_p(a), _p(out), n, st)
     elif op == "scale":

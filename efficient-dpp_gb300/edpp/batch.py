@@ -18,7 +18,7 @@ from pathlib import Path
 
 import numpy as np
 
-from . import _p, _torch, check, current_stream_handle, lib, workspace
+from . import _p, _stream, _torch, check, current_stream_handle, lib, workspace
 
 SEG_DTYPE = np.dtype([("offset", "<i8"), ("length", "<i4"), ("op", "<i4"), ("buckets", "<i4"),
                       ("reserved", "<i4")])
@@ -156,7 +156,7 @@ class Plan:
 
     def launch(self, in0, in1, out0, out1, ws):
         check(lib().edpp_batch_launch(self.h, _p(in0), _p(in1), _p(out0), _p(out1), _p(ws),
-                                      ws.numel(), current_stream_handle()), "batch_launch")
+                                      ws.numel(), _stream()), "batch_launch")
 
 
 def plain_workspace(segs, device=None):
