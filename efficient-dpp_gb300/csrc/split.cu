@@ -20,7 +20,7 @@
 //              tile is re-laid out in shared memory in bucket order, and
 //              written out as one contiguous run per bucket (coalesced), at
 //              his[b*T + t] + rank.  Few buckets rank by votes or per-warp lane
-//              masks and re-lay the elements out (below); from 8 to 64 buckets
+//              masks and re-lay the elements out (below); from 8 to 32 buckets
 //              on, depending on the layout, one atomic per element ranks and
 //              only source positions are re-laid out (split_index.cuh).
 //
@@ -66,7 +66,7 @@ template <int LAYOUT> __device__ __forceinline__ int32_t key_at(const int32_t *k
 }
 
 // ---- stage 1: per-tile bucket counts ----------------------------------------
-template <int LAYOUT>
+template <int LAYOUT, int TILE>
 __global__ void __launch_bounds__(kHistThreads)
     split_hist_kernel(const int32_t *__restrict__ keys, int64_t n, int buckets, int shift,
                       int64_t tiles, int32_t *__restrict__ his, bool vec) {
@@ -75,29 +75,29 @@ __global__ void __launch_bounds__(kHistThreads)
   for (int b = threadIdx.x; b < buckets; b += kHistThreads) cnt[b] = 0;
   __syncthreads();
   const int64_t t = blockIdx.x;
-  const int64_t base = t * kTile;
-  const int count = static_cast<int>(min64(kTile, n - base));
+  const int64_t base = t * TILE;
+  const int count = static_cast<int>(min64(TILE, n - base));
 
   auto add = [&](bool valid, int32_t key) {
     if (valid) atomicAdd(&cnt[(static_cast<unsigned>(key) >> shift) & mask], 1u);
   };
 
-  if (LAYOUT != EDPP_KVS_AOS && vec && count == kTile) {
+  if (LAYOUT != EDPP_KVS_AOS && vec && count == TILE) {
     // 16-byte vectors, warp-contiguous: 4 keys per thread per step.
     const int4 *k4 = reinterpret_cast<const int4 *>(keys + base);
 #pragma unroll 2
-    for (int v = threadIdx.x; v < kTile / 4; v += kHistThreads) {
+    for (int v = threadIdx.x; v < TILE / 4; v += kHistThreads) {
       const int4 q = __ldcs(k4 + v);
       add(true, q.x);
       add(true, q.y);
       add(true, q.z);
       add(true, q.w);
     }
-  } else if (LAYOUT == EDPP_KVS_AOS && vec && count == kTile) {
+  } else if (LAYOUT == EDPP_KVS_AOS && vec && count == TILE) {
     // 16-byte vectors of two pairs.
     const int4 *p4 = reinterpret_cast<const int4 *>(keys + 2 * base);
 #pragma unroll 2
-    for (int v = threadIdx.x; v < kTile / 2; v += kHistThreads) {
+    for (int v = threadIdx.x; v < TILE / 2; v += kHistThreads) {
       const int4 q = __ldcs(p4 + v);
       add(true, q.x);
       add(true, q.z);
@@ -592,11 +592,25 @@ size_t his_bytes(int64_t tiles, int buckets) {
 
 // From this many buckets on the scatter stages positions (split_index.cuh).
 // Whole split of 2^28 elements, element staging against position staging (ms):
-// KVS_SOA 16 buckets 1.144 / 1.138, 32 1.232 / 1.116, 256 1.513 / 1.242;
-// KVS_AOS 8 buckets 1.370 / 1.326, 256 1.590 / 1.339; KO 32 buckets 0.974 /
-// 0.986, 64 1.009 / 0.989, 256 1.233 / 1.092.
+// KVS_SOA 8 buckets 1.125 / 1.124, 16 1.143 / 1.044, 64 1.276 / 1.014, 256 1.513
+// / 1.207; KVS_AOS 4 buckets 1.358 / 1.439, 8 1.370 / 1.266, 256 1.590 / 1.338;
+// KO 16 buckets 0.907 / 0.905, 32 0.974 / 0.873, 256 1.233 / 1.009.
 template <int LAYOUT> constexpr int index_buckets() {
-  return LAYOUT == EDPP_KO ? 64 : LAYOUT == EDPP_KVS_SOA ? 32 : 8;
+  return LAYOUT == EDPP_KO ? 32 : LAYOUT == EDPP_KVS_SOA ? 16 : 8;
+}
+
+// Position staging of pairs up to 64 buckets takes tiles of 6144, of which
+// three fit an SM (70 KB each) where two of 8192 do: 2^28 pairs, 64 buckets
+// 1.117 -> 1.014 ms.  With more buckets the shorter runs and the larger
+// histogram cost more than that gains: 128 buckets 1.150 against 1.128, 256
+// 1.344 against 1.207.
+constexpr int kPairTile = 6144, kPairTileBuckets = 64;
+template <int LAYOUT> bool pair_tile(int buckets) {
+  return LAYOUT != EDPP_KO && buckets >= index_buckets<LAYOUT>() && buckets <= kPairTileBuckets;
+}
+// Tile of the three-launch split.
+template <int LAYOUT> int split_tile(int buckets) {
+  return pair_tile<LAYOUT>(buckets) ? kPairTile : kTile;
 }
 
 // Dynamic shared-memory limit of `kernel` raised to `bytes`, once per device;
@@ -659,26 +673,30 @@ template <int LAYOUT> bool bulk_runs(const SplitArgs &a) {
          aligned16(a.keys_out) && (LAYOUT != EDPP_KVS_SOA || aligned16(a.vals_out));
 }
 
+template <int LAYOUT, int TILE>
+int launch_index(const SplitArgs &a, int64_t tiles, const int32_t *his, cudaStream_t st) {
+  constexpr auto kernel = split_index_kernel<LAYOUT, TILE, false>;
+  const int s =
+      prepare_kernel<kernel>(kIndexThreads, index_smem_bytes<LAYOUT, TILE>(kOnePassMax), nullptr);
+  if (s != EDPP_OK) return s;
+  kernel<<<static_cast<unsigned>(tiles), kIndexThreads, index_smem_bytes<LAYOUT, TILE>(a.buckets),
+           st>>>(a.keys_in, a.keys_out, a.vals_in, a.vals_out, a.n, a.buckets, a.shift, tiles, his,
+                 a.tma, a.exact, kDefaultWaitNs, fault_word(), FusedArgs{});
+  return launch_status();
+}
+
 template <int LAYOUT>
 int launch_scatter(const SplitArgs &a, int64_t tiles, const int32_t *his, cudaStream_t st) {
-  const unsigned grid = static_cast<unsigned>(tiles);
-  if (a.buckets >= index_buckets<LAYOUT>()) {
-    constexpr auto kernel = split_index_kernel<LAYOUT, kTile, false>;
-    const int s = prepare_kernel<kernel>(
-        kIndexThreads, index_smem_bytes<LAYOUT, kTile>(kOnePassMax), nullptr);
-    if (s != EDPP_OK) return s;
-    kernel<<<grid, kIndexThreads, index_smem_bytes<LAYOUT, kTile>(a.buckets), st>>>(
-        a.keys_in, a.keys_out, a.vals_in, a.vals_out, a.n, a.buckets, a.shift, tiles, his, a.tma,
-        a.exact, kDefaultWaitNs, fault_word(), FusedArgs{});
-    return launch_status();
-  }
+  if (pair_tile<LAYOUT>(a.buckets))
+    return launch_index<LAYOUT, LAYOUT == EDPP_KO ? kTile : kPairTile>(a, tiles, his, st);
+  if (a.buckets >= index_buckets<LAYOUT>()) return launch_index<LAYOUT, kTile>(a, tiles, his, st);
   constexpr auto kernel = split_scatter_kernel<kScatterThreads, LAYOUT, kTile, false>;
   const int s = prepare_kernel<kernel>(
       kScatterThreads, scatter_smem_bytes<kScatterThreads, LAYOUT, kTile>(index_buckets<LAYOUT>(), true),
       nullptr);
   if (s != EDPP_OK) return s;
   const bool bulk = bulk_runs<LAYOUT>(a);
-  kernel<<<grid, kScatterThreads, scatter_smem_bytes<kScatterThreads, LAYOUT, kTile>(a.buckets, bulk),
+  kernel<<<static_cast<unsigned>(tiles), kScatterThreads, scatter_smem_bytes<kScatterThreads, LAYOUT, kTile>(a.buckets, bulk),
            st>>>(a.keys_in, a.keys_out, a.vals_in, a.vals_out, a.n, a.buckets, a.shift, tiles, his,
                  a.tma, bulk, kDefaultWaitNs, fault_word(), FusedArgs{});
   return launch_status();
@@ -766,7 +784,8 @@ int split_layout(const int32_t *keys_in, int32_t *keys_out, int32_t *bucket_star
                  int buckets, const int32_t *vals_in, int32_t *vals_out, void *ws, size_t ws_bytes,
                  cudaStream_t st, int shift = 0, bool exact = false) {
   if (buckets > kOnePassMax) return EDPP_EINVAL;  // callers take two passes from 2048 on
-  const int64_t tiles = (n + kTile - 1) / kTile;
+  const int tile = split_tile<LAYOUT>(buckets);
+  const int64_t tiles = (n + tile - 1) / tile;
   int32_t *his = static_cast<int32_t *>(ws);
   const int64_t hlen = tiles * buckets;
   void *scan_ws = static_cast<char *>(ws) + his_bytes(tiles, buckets);
@@ -775,8 +794,9 @@ int split_layout(const int32_t *keys_in, int32_t *keys_out, int32_t *bucket_star
                     aligned16(keys_in) && (LAYOUT != EDPP_KVS_SOA || aligned16(vals_in)), exact};
   int s = split_fused<LAYOUT>(a, static_cast<char *>(ws), st);
   if (s != EDPP_ENOMEM) return s;
-  split_hist_kernel<LAYOUT><<<static_cast<unsigned>(tiles), kHistThreads, 0, st>>>(
-      keys_in, n, buckets, shift, tiles, his, aligned16(keys_in));
+  const auto hist = tile == kTile ? split_hist_kernel<LAYOUT, kTile> : split_hist_kernel<LAYOUT, kPairTile>;
+  hist<<<static_cast<unsigned>(tiles), kHistThreads, 0, st>>>(keys_in, n, buckets, shift, tiles, his,
+                                                              aligned16(keys_in));
   s = launch_status();
   if (s != EDPP_OK) return s;
   s = edpp_scan_exclusive_i32(his, his, hlen, EDPP_SCAN_LOOKBACK, scan_ws, scan_ws_bytes, st);
@@ -797,7 +817,9 @@ int split_layout(const int32_t *keys_in, int32_t *keys_out, int32_t *bucket_star
 constexpr int kLsdBuckets = 2048;
 
 size_t split_pass_ws_bytes(int64_t n, int buckets) {
-  const int64_t tiles = (n + kTile - 1) / kTile;
+  // enough for every layout's tile
+  const int64_t tile = buckets <= kPairTileBuckets ? kPairTile : kTile;
+  const int64_t tiles = (n + tile - 1) / tile;
   return std::max(his_bytes(tiles, buckets) +
                       edpp_scan_workspace_size(tiles * buckets, EDPP_I32, EDPP_SCAN_LOOKBACK),
                   fused_ws_bytes(n, buckets));

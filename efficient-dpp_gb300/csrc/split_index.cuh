@@ -16,9 +16,9 @@
 // (the returning atomic 8, the random reads of key and value 7, the position
 // store and the slot lookup 3 each) against 34 for per-warp lane masks with
 // the pairs themselves re-laid out, and nothing in the ranking waits for the
-// step before.  Scatter alone, 2^28 pairs, 256 buckets: 1.30 -> 1.03 ms; whole
+// step before.  Scatter alone, 2^28 pairs, 256 buckets: 1.30 -> 1.00 ms; whole
 // splits at index_buckets() in split.cu.  512 and 1024 buckets ranked by a
-// leader table before: 1.85 -> 1.51 and 2.57 -> 2.21 ms.
+// leader table before: 1.85 -> 1.51 and 2.57 -> 2.19 ms.
 #pragma once
 
 namespace edpp {
@@ -38,8 +38,15 @@ template <int LAYOUT, int TILE> size_t index_smem_bytes(int buckets) {
          8 * static_cast<size_t>(buckets);
 }
 
+// Blocks per SM: three where shared memory holds them (40 registers), else two.
+// 2^28 keys, 64 / 256 buckets, two against three: 0.989 -> 0.872, 1.090 -> 1.009
+// ms.  The fused form has one or two blocks per SM to run anyway.
+template <int LAYOUT, int TILE, bool kFused> constexpr int index_blocks() {
+  return !kFused && (LAYOUT == EDPP_KO || TILE < 8192) ? 3 : 2;
+}
+
 template <int LAYOUT, int TILE, bool kFused>
-__global__ void __launch_bounds__(kIndexThreads, 2)
+__global__ void __launch_bounds__(kIndexThreads, index_blocks<LAYOUT, TILE, kFused>())
     split_index_kernel(const int32_t *__restrict__ keys_in, int32_t *__restrict__ keys_out,
                        const int32_t *__restrict__ vals_in, int32_t *__restrict__ vals_out,
                        int64_t n, int buckets, int shift, int64_t tiles,
@@ -186,7 +193,10 @@ __global__ void __launch_bounds__(kIndexThreads, 2)
   // -- write out: consecutive threads write consecutive slots of a bucket run --
   auto write_out = [&]() {
     bool bad = false;
-#pragma unroll 4
+    // 8192 pairs, 256 buckets: four at once 1.243, two 1.210 ms at 2^28; the
+    // other forms prefer four (6144 pairs 1.013 against 1.054 with one)
+    constexpr int kUnroll = LAYOUT == EDPP_KVS_SOA && TILE == 8192 ? 2 : 4;
+#pragma unroll kUnroll
     for (int s0 = 0; s0 < TILE; s0 += THREADS) {
       const int s = s0 + tid;
       const bool valid = s < count;

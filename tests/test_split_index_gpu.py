@@ -1,4 +1,4 @@
-"""The position-staged split (from 8, 32 or 64 buckets on, by layout) at tile
+"""The position-staged split (from 8, 16 or 32 buckets on, by layout) at tile
 edges, in both of its rankings: the quick one with its check, and the exact one
 that a tile takes when the check fails; skewed keys, every key in one bucket,
 one launch and three launches."""
@@ -37,11 +37,11 @@ def _split(edpp, torch, keys, vals, buckets, layout, exact):
 
 @pytest.mark.parametrize("exact", [False, True])
 @pytest.mark.parametrize("layout", ["ko", "soa", "aos"])
-@pytest.mark.parametrize("buckets", [8, 32, 64, 256, 512, 1024])
+@pytest.mark.parametrize("buckets", [8, 16, 32, 64, 128, 256, 512, 1024])
 def test_both_rankings(cuda, edpp, buckets, layout, exact):
     g = cuda.Generator(device="cuda")
     # one launch up to 2.4 million elements, three launches above
-    for n in (1, 33, 8191, 8193, 100_003, (1 << 22) + 8192, (1 << 22) + 4099):
+    for n in (1, 33, 6143, 6145, 8191, 8193, 100_003, (1 << 22) + 8192, 6144 * 700, 6144 * 700 + 1):
         g.manual_seed(n + buckets)
         vals = cuda.arange(n, device="cuda", dtype=cuda.int32)
         uniform = cuda.randint(-2**31, 2**31 - 1, (n,), generator=g, device="cuda", dtype=cuda.int32)
