@@ -1,0 +1,113 @@
+// pos_stage.cuh — ranking and re-layout of a split tile by source positions,
+// shared by the split (split_index.cuh) and the batched split tiles (batch.cu).
+//
+// A tile stays in shared memory as loaded.  Ranking takes one shared-memory
+// atomic per element: the old value of the (warp, bucket) counter is the
+// element's rank among its warp's elements of the bucket.  What is re-laid out
+// in bucket order is only the 16-bit source position; the write-out fetches key
+// and value from there.
+//
+// Atomics of one warp instruction on one counter, and of successive
+// instructions, have returned in lane and program order wherever it was
+// looked at, but nothing promises that, so the write-out checks it: positions
+// must ascend within every bucket's run.  A tile that fails is ranked again by
+// peer groups (exact, slow) and written over.
+//
+// The counters are 16 bits, cnt16[warp * buckets + b], an even number of
+// buckets; between rank() and place() the caller turns them into each warp's
+// first slot of the bucket.  Callers put barriers between the steps.
+#pragma once
+
+#include "common.cuh"
+
+namespace edpp {
+
+template <int NT, int TILE> struct PosStage {
+  static constexpr int kWarps = NT / 32;
+  static constexpr int kSeg = TILE / kWarps;  // a warp's contiguous part of the tile
+  static constexpr int kIters = kSeg / 32;
+
+  __device__ __forceinline__ static int position(int it) {
+    return static_cast<int>(threadIdx.x >> 5) * kSeg + it * 32 + static_cast<int>(threadIdx.x & 31);
+  }
+
+  // br[it] = bucket | rank << 16 of this lane's elements; bucket_at(position).
+  template <typename F>
+  __device__ __forceinline__ static void rank(uint16_t *cnt16, int buckets, int count, F bucket_at,
+                                              uint32_t (&br)[kIters]) {
+    // two counters per 32-bit word
+    uint32_t *words =
+        reinterpret_cast<uint32_t *>(cnt16) + (threadIdx.x >> 5) * (static_cast<unsigned>(buckets) >> 1);
+#pragma unroll
+    for (int it = 0; it < kIters; ++it) {
+      const int pos = position(it);
+      br[it] = pos < count ? static_cast<uint32_t>(bucket_at(pos)) : 0u;
+    }
+#pragma unroll
+    for (int it = 0; it < kIters; ++it) {
+      const uint32_t sh = (br[it] & 1u) * 16u;
+      if (position(it) < count)
+        br[it] |= ((atomicAdd(&words[br[it] >> 1], 1u << sh) >> sh) & 0xffffu) << 16;
+    }
+  }
+
+  __device__ __forceinline__ static void place(const uint16_t *cnt16, int buckets, int count,
+                                               const uint32_t (&br)[kIters], uint16_t *s_pos) {
+    const uint16_t *mine = cnt16 + (threadIdx.x >> 5) * buckets;
+#pragma unroll
+    for (int it = 0; it < kIters; ++it) {
+      const int pos = position(it);
+      if (pos < count) s_pos[mine[br[it] & 0xffffu] + (br[it] >> 16)] = static_cast<uint16_t>(pos);
+    }
+  }
+
+  // Exact slots, instead of place(): the lanes of a bucket count their lower
+  // peers, step by step in input order, advancing the warp's slot of the bucket.
+  template <typename F>
+  __device__ __forceinline__ static void place_exact(uint16_t *cnt16, int buckets, int count,
+                                                     F bucket_at, uint16_t *s_pos) {
+    uint16_t *mine = cnt16 + (threadIdx.x >> 5) * buckets;
+    unsigned lt;
+    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
+    for (int it = 0; it < kIters; ++it) {
+      const int pos = position(it);
+      const bool valid = pos < count;
+      const int b = valid ? bucket_at(pos) : 0;
+      const unsigned vmask = __ballot_sync(0xffffffffu, valid);
+      const unsigned peers = match_low_bits(static_cast<unsigned>(b), 31 - __clz(buckets), vmask);
+      const int before = valid ? mine[b] : 0;
+      __syncwarp();
+      if (valid && (peers & lt) == 0u) mine[b] = static_cast<uint16_t>(before + __popc(peers));
+      __syncwarp();
+      if (valid) s_pos[before + __popc(peers & lt)] = static_cast<uint16_t>(pos);
+    }
+  }
+
+  // store(slot, bucket, load(position)) for every slot, consecutive threads on
+  // consecutive slots; bucket_of(element).  True when a position is out of order.
+  template <int UNROLL, typename L, typename B, typename S>
+  __device__ __forceinline__ static bool write_out(const uint16_t *s_pos, int count, L load,
+                                                   B bucket_of, S store) {
+    const int lane = threadIdx.x & 31;
+    bool bad = false;
+#pragma unroll UNROLL
+    for (int s0 = 0; s0 < TILE; s0 += NT) {
+      const int s = s0 + static_cast<int>(threadIdx.x);
+      const bool valid = s < count;
+      const int pos = valid ? s_pos[s] : 0;
+      const auto e = load(pos);
+      const int b = bucket_of(e);
+      const int mine = b * TILE + pos;  // ascends from slot to slot
+      int before = __shfl_up_sync(0xffffffffu, mine, 1);
+      if (lane == 0 && valid) {
+        const int q = s > 0 ? s_pos[s - 1] : 0;
+        before = s > 0 ? bucket_of(load(q)) * TILE + q : -1;
+      }
+      bad |= valid && before >= mine;
+      if (valid) store(s, b, e);
+    }
+    return bad;
+  }
+};
+
+}  // namespace edpp

@@ -1,16 +1,6 @@
 // split_index.cuh — split scatter that stages source positions (split.cu).
 //
-// A tile stays in shared memory as loaded.  Ranking takes one shared-memory
-// atomic per element: the old value of the (warp, bucket) counter is the
-// element's rank among its warp's elements of the bucket.  What is re-laid out
-// in bucket order is only the 16-bit source position; the write-out fetches key
-// and value from there.
-//
-// Atomics of one warp instruction on one counter, and of successive
-// instructions, have returned in lane and program order wherever it was
-// looked at, but nothing promises that, so the write-out checks it: positions
-// must ascend within every bucket's run.  A tile that fails is ranked again by
-// peer groups (exact, slow) and written over.
+// Ranking, re-layout and write-out as pos_stage.cuh describes them.
 //
 // Bound by the shared-memory pipe: 27 wavefronts per 32 pairs at 256 buckets
 // (the returning atomic 8, the random reads of key and value 7, the position
@@ -21,20 +11,16 @@
 // leader table before: 1.85 -> 1.51 and 2.57 -> 2.19 ms.
 #pragma once
 
+#include "pos_stage.cuh"
+
 namespace edpp {
 namespace {
 
 constexpr int kIndexThreads = 512;
-template <int TILE> struct IndexCfg {
-  static constexpr int kWarps = kIndexThreads / 32;
-  static constexpr int kSeg = TILE / kWarps;
-  static constexpr int kIters = kSeg / 32;
-};
-
 // tile | positions | counters of 16 bits per (warp, bucket) | totals | run starts
 template <int LAYOUT, int TILE> size_t index_smem_bytes(int buckets) {
   return static_cast<size_t>(TILE) * (LAYOUT == EDPP_KO ? 4 : 8) + 2 * static_cast<size_t>(TILE) +
-         round_up(static_cast<size_t>(IndexCfg<TILE>::kWarps) * buckets * 2, 16) +
+         round_up(static_cast<size_t>(kIndexThreads / 32) * buckets * 2, 16) +
          8 * static_cast<size_t>(buckets);
 }
 
@@ -52,7 +38,7 @@ __global__ void __launch_bounds__(kIndexThreads, index_blocks<LAYOUT, TILE, kFus
                        int64_t n, int buckets, int shift, int64_t tiles,
                        const int32_t *__restrict__ his, bool tma, bool exact, uint64_t timeout_ns,
                        unsigned *fault, FusedArgs fused) {
-  using C = IndexCfg<TILE>;
+  using C = PosStage<kIndexThreads, TILE>;
   constexpr int THREADS = kIndexThreads;
   extern __shared__ __align__(128) unsigned char smem[];
   int32_t *s_keys = reinterpret_cast<int32_t *>(smem);
@@ -97,9 +83,8 @@ __global__ void __launch_bounds__(kIndexThreads, index_blocks<LAYOUT, TILE, kFus
       if (LAYOUT == EDPP_KVS_SOA) s_vals[i] = vals_in[base + i];
     }
   }
-  uint32_t *cnt_words = reinterpret_cast<uint32_t *>(cnt16);  // two counters per word
-  const int row = buckets / 2;                                // words per warp
-  for (int i = tid; i < C::kWarps * row; i += THREADS) cnt_words[i] = 0u;
+  for (int i = tid; i < C::kWarps * buckets / 2; i += THREADS)
+    reinterpret_cast<uint32_t *>(cnt16)[i] = 0u;
   const int per = (buckets + THREADS - 1) / THREADS;
   const int b_lo = min(buckets, tid * per), b_hi = min(buckets, b_lo + per);
   constexpr int kHisPre = 2;  // 512 threads serve up to 1024 buckets
@@ -112,26 +97,20 @@ __global__ void __launch_bounds__(kIndexThreads, index_blocks<LAYOUT, TILE, kFus
     if (!mbar_wait_bounded(&bar, 0, timeout_ns, fault)) return;
   }
   __syncthreads();
-  auto key_of = [&](int pos) { return LAYOUT == EDPP_KVS_AOS ? s_pairs[pos].x : s_keys[pos]; };
-  auto bucket_of = [&](int32_t key) {
-    return static_cast<int>((static_cast<unsigned>(key) >> shift) & mask);
+  // an element: {key, value}, or the key alone
+  auto load = [&](int pos) {
+    if constexpr (LAYOUT == EDPP_KVS_AOS) return s_pairs[pos];
+    else if constexpr (LAYOUT == EDPP_KVS_SOA) return make_int2(s_keys[pos], s_vals[pos]);
+    else return make_int2(s_keys[pos], 0);
   };
-
-  // -- rank: warp w owns tile positions [w*kSeg, (w+1)*kSeg), in order --
-  uint32_t br[C::kIters];  // bucket | rank << 16
-  uint32_t *my_words = cnt_words + w * row;
-#pragma unroll
-  for (int it = 0; it < C::kIters; ++it) {
-    const int pos = w * C::kSeg + it * 32 + lane;
-    br[it] = pos < count ? static_cast<uint32_t>(bucket_of(key_of(pos))) : 0u;
-  }
-#pragma unroll
-  for (int it = 0; it < C::kIters; ++it) {
-    const int pos = w * C::kSeg + it * 32 + lane;
-    const uint32_t sh = (br[it] & 1u) * 16u;
-    if (pos < count)
-      br[it] |= ((atomicAdd(&my_words[br[it] >> 1], 1u << sh) >> sh) & 0xffffu) << 16;
-  }
+  auto bucket_of = [&](int2 e) {
+    return static_cast<int>((static_cast<unsigned>(e.x) >> shift) & mask);
+  };
+  auto bucket_at = [&](int pos) {
+    return bucket_of(make_int2(LAYOUT == EDPP_KVS_AOS ? s_pairs[pos].x : s_keys[pos], 0));
+  };
+  uint32_t br[C::kIters];
+  C::rank(cnt16, buckets, count, bucket_at, br);
   __syncthreads();
 
   // -- per bucket: tile count, tile offset, then each warp's first slot
@@ -179,79 +158,30 @@ __global__ void __launch_bounds__(kIndexThreads, index_blocks<LAYOUT, TILE, kFus
   }
   __syncthreads();
 
-  // -- positions in bucket order --
-  if (!exact) {
-#pragma unroll
-    for (int it = 0; it < C::kIters; ++it) {
-      const int pos = w * C::kSeg + it * 32 + lane;
-      if (pos < count)
-        s_pos[cnt16[w * buckets + (br[it] & 0xffffu)] + (br[it] >> 16)] = static_cast<uint16_t>(pos);
+  // -- re-lay out and write --
+  auto store = [&](int slot, int b, int2 e) {
+    const int64_t o = static_cast<int64_t>(gofs[b]) + slot;
+    if (LAYOUT == EDPP_KVS_AOS) {
+      reinterpret_cast<int2 *>(keys_out)[o] = e;
+    } else {
+      keys_out[o] = e.x;
+      if (LAYOUT == EDPP_KVS_SOA) vals_out[o] = e.y;
     }
-    __syncthreads();
-  }
-
-  // -- write out: consecutive threads write consecutive slots of a bucket run --
-  auto write_out = [&]() {
-    bool bad = false;
-    // 8192 pairs, 256 buckets: four at once 1.243, two 1.210 ms at 2^28; the
-    // other forms prefer four (6144 pairs 1.013 against 1.054 with one)
-    constexpr int kUnroll = LAYOUT == EDPP_KVS_SOA && TILE == 8192 ? 2 : 4;
-#pragma unroll kUnroll
-    for (int s0 = 0; s0 < TILE; s0 += THREADS) {
-      const int s = s0 + tid;
-      const bool valid = s < count;
-      const int pos = valid ? s_pos[s] : 0;
-      int32_t key = 0, val = 0;
-      if (LAYOUT == EDPP_KVS_AOS) {
-        const int2 p = s_pairs[pos];
-        key = p.x;
-        val = p.y;
-      } else {
-        key = s_keys[pos];
-        if (LAYOUT == EDPP_KVS_SOA) val = s_vals[pos];
-      }
-      const int b = bucket_of(key);
-      // (bucket, position) ascends from slot to slot
-      const int mine = b * TILE + pos;
-      int before = __shfl_up_sync(0xffffffffu, mine, 1);
-      if (lane == 0 && valid) {
-        const int q = s > 0 ? s_pos[s - 1] : 0;
-        before = s > 0 ? bucket_of(key_of(q)) * TILE + q : -1;
-      }
-      bad |= valid && before >= mine;
-      if (valid) {
-        const int64_t o = static_cast<int64_t>(gofs[b]) + s;
-        if (LAYOUT == EDPP_KVS_AOS) {
-          reinterpret_cast<int2 *>(keys_out)[o] = make_int2(key, val);
-        } else {
-          keys_out[o] = key;
-          if (LAYOUT == EDPP_KVS_SOA) vals_out[o] = val;
-        }
-      }
-    }
-    return bad;
   };
+  // 8192 pairs, 256 buckets: four elements in flight per thread 1.243, two 1.210
+  // ms at 2^28; the other forms prefer four (6144 pairs 1.013 against 1.054 with
+  // one)
+  constexpr int kUnroll = LAYOUT == EDPP_KVS_SOA && TILE == 8192 ? 2 : 4;
   bool bad = exact;
-  if (!exact) bad = write_out();
-  if (__syncthreads_or(bad)) {
-    // exact ranks: the lanes of a bucket count their lower peers, warp by warp
-    // in input order, advancing the warp's slot of the bucket
-    const unsigned lt = lanemask_lt();
-    for (int it = 0; it < C::kIters; ++it) {
-      const int pos = w * C::kSeg + it * 32 + lane;
-      const bool valid = pos < count;
-      const int b = valid ? bucket_of(key_of(pos)) : 0;
-      const unsigned vmask = __ballot_sync(0xffffffffu, valid);
-      const unsigned peers = match_low_bits(static_cast<unsigned>(b), 31 - __clz(buckets), vmask);
-      const int before = valid ? cnt16[w * buckets + b] : 0;
-      __syncwarp();
-      if (valid && (peers & lt) == 0u)
-        cnt16[w * buckets + b] = static_cast<uint16_t>(before + __popc(peers));
-      __syncwarp();
-      if (valid) s_pos[before + __popc(peers & lt)] = static_cast<uint16_t>(pos);
-    }
+  if (!exact) {
+    C::place(cnt16, buckets, count, br, s_pos);
     __syncthreads();
-    write_out();
+    bad = C::template write_out<kUnroll>(s_pos, count, load, bucket_of, store);
+  }
+  if (__syncthreads_or(bad)) {
+    C::place_exact(cnt16, buckets, count, bucket_at, s_pos);
+    __syncthreads();
+    C::template write_out<1>(s_pos, count, load, bucket_of, store);
   }
 }
 
