@@ -66,52 +66,71 @@ template <int LAYOUT> __device__ __forceinline__ int32_t key_at(const int32_t *k
 }
 
 // ---- stage 1: per-tile bucket counts ----------------------------------------
-template <int LAYOUT, int TILE>
+// One block counts TP consecutive tiles.  Row b of his is `stride` long, tiles
+// rounded up to TP (the padding columns count zero).  Bound by DRAM up to 64
+// buckets; above, one 4-byte store per bucket and tile cost as much as the
+// reading (2^28 keys: 64 buckets 0.159, 256 0.194, 1024 0.337 ms), so large
+// inputs take four tiles per block and 16-byte stores: 0.153, 0.164 and 0.214
+// ms; 2^26 keys, 256 buckets 0.054 -> 0.047.
+template <int LAYOUT, int TILE, int TP>
 __global__ void __launch_bounds__(kHistThreads)
     split_hist_kernel(const int32_t *__restrict__ keys, int64_t n, int buckets, int shift,
-                      int64_t tiles, int32_t *__restrict__ his, bool vec) {
-  __shared__ uint32_t cnt[kOnePassMax];
+                      int64_t stride, int32_t *__restrict__ his, bool vec) {
+  static_assert(TP == 1 || TP == 4, "a 4- or 16-byte store per bucket");
+  __shared__ uint32_t cnt[TP * kOnePassMax];  // [tile][bucket]
   const unsigned mask = static_cast<unsigned>(buckets - 1);
-  for (int b = threadIdx.x; b < buckets; b += kHistThreads) cnt[b] = 0;
+  for (int b = threadIdx.x; b < TP * buckets; b += kHistThreads) cnt[b] = 0;
   __syncthreads();
-  const int64_t t = blockIdx.x;
-  const int64_t base = t * TILE;
-  const int count = static_cast<int>(min64(TILE, n - base));
-
-  auto add = [&](bool valid, int32_t key) {
-    if (valid) atomicAdd(&cnt[(static_cast<unsigned>(key) >> shift) & mask], 1u);
-  };
-
-  if (LAYOUT != EDPP_KVS_AOS && vec && count == TILE) {
-    // 16-byte vectors, warp-contiguous: 4 keys per thread per step.
-    const int4 *k4 = reinterpret_cast<const int4 *>(keys + base);
+  const int64_t t0 = static_cast<int64_t>(blockIdx.x) * TP;
+#pragma unroll 1
+  for (int j = 0; j < TP; ++j) {
+    const int64_t base = (t0 + j) * TILE;
+    if (base >= n) break;
+    const int count = static_cast<int>(min64(TILE, n - base));
+    uint32_t *mine = cnt + j * buckets;
+    auto add = [&](bool valid, int32_t key) {
+      if (valid) atomicAdd(&mine[(static_cast<unsigned>(key) >> shift) & mask], 1u);
+    };
+    if (LAYOUT != EDPP_KVS_AOS && vec && count == TILE) {
+      // 16-byte vectors, warp-contiguous: 4 keys per thread per step.
+      const int4 *k4 = reinterpret_cast<const int4 *>(keys + base);
 #pragma unroll 2
-    for (int v = threadIdx.x; v < TILE / 4; v += kHistThreads) {
-      const int4 q = __ldcs(k4 + v);
-      add(true, q.x);
-      add(true, q.y);
-      add(true, q.z);
-      add(true, q.w);
-    }
-  } else if (LAYOUT == EDPP_KVS_AOS && vec && count == TILE) {
-    // 16-byte vectors of two pairs.
-    const int4 *p4 = reinterpret_cast<const int4 *>(keys + 2 * base);
+      for (int v = threadIdx.x; v < TILE / 4; v += kHistThreads) {
+        const int4 q = __ldcs(k4 + v);
+        add(true, q.x);
+        add(true, q.y);
+        add(true, q.z);
+        add(true, q.w);
+      }
+    } else if (LAYOUT == EDPP_KVS_AOS && vec && count == TILE) {
+      // 16-byte vectors of two pairs.
+      const int4 *p4 = reinterpret_cast<const int4 *>(keys + 2 * base);
 #pragma unroll 2
-    for (int v = threadIdx.x; v < TILE / 2; v += kHistThreads) {
-      const int4 q = __ldcs(p4 + v);
-      add(true, q.x);
-      add(true, q.z);
-    }
-  } else {
-    for (int i0 = 0; i0 < count; i0 += kHistThreads) {
-      const int i = i0 + threadIdx.x;
-      const bool valid = i < count;
-      add(valid, valid ? key_at<LAYOUT>(keys, base + i) : 0);
+      for (int v = threadIdx.x; v < TILE / 2; v += kHistThreads) {
+        const int4 q = __ldcs(p4 + v);
+        add(true, q.x);
+        add(true, q.z);
+      }
+    } else {
+      for (int i0 = 0; i0 < count; i0 += kHistThreads) {
+        const int i = i0 + threadIdx.x;
+        const bool valid = i < count;
+        add(valid, valid ? key_at<LAYOUT>(keys, base + i) : 0);
+      }
     }
   }
   __syncthreads();
-  for (int b = threadIdx.x; b < buckets; b += kHistThreads)
-    his[static_cast<int64_t>(b) * tiles + t] = static_cast<int32_t>(cnt[b]);
+  for (int b = threadIdx.x; b < buckets; b += kHistThreads) {
+    int32_t *dst = his + static_cast<int64_t>(b) * stride + t0;
+    if (TP == 4) {
+      int32_t c[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) c[j] = static_cast<int32_t>(cnt[(TP == 4 ? j : 0) * buckets + b]);
+      *reinterpret_cast<int4 *>(dst) = make_int4(c[0], c[1], c[2], c[3]);
+    } else {
+      *dst = static_cast<int32_t>(cnt[b]);
+    }
+  }
 }
 
 // ---- stage 3: stable scatter --------------------------------------------------
@@ -674,22 +693,25 @@ template <int LAYOUT> bool bulk_runs(const SplitArgs &a) {
 }
 
 template <int LAYOUT, int TILE>
-int launch_index(const SplitArgs &a, int64_t tiles, const int32_t *his, cudaStream_t st) {
+int launch_index(const SplitArgs &a, int64_t tiles, int64_t stride, const int32_t *his,
+                 cudaStream_t st) {
   constexpr auto kernel = split_index_kernel<LAYOUT, TILE, false>;
   const int s =
       prepare_kernel<kernel>(kIndexThreads, index_smem_bytes<LAYOUT, TILE>(kOnePassMax), nullptr);
   if (s != EDPP_OK) return s;
   kernel<<<static_cast<unsigned>(tiles), kIndexThreads, index_smem_bytes<LAYOUT, TILE>(a.buckets),
-           st>>>(a.keys_in, a.keys_out, a.vals_in, a.vals_out, a.n, a.buckets, a.shift, tiles, his,
+           st>>>(a.keys_in, a.keys_out, a.vals_in, a.vals_out, a.n, a.buckets, a.shift, stride, his,
                  a.tma, a.exact, kDefaultWaitNs, fault_word(), FusedArgs{});
   return launch_status();
 }
 
 template <int LAYOUT>
-int launch_scatter(const SplitArgs &a, int64_t tiles, const int32_t *his, cudaStream_t st) {
+int launch_scatter(const SplitArgs &a, int64_t tiles, int64_t stride, const int32_t *his,
+                   cudaStream_t st) {
   if (pair_tile<LAYOUT>(a.buckets))
-    return launch_index<LAYOUT, LAYOUT == EDPP_KO ? kTile : kPairTile>(a, tiles, his, st);
-  if (a.buckets >= index_buckets<LAYOUT>()) return launch_index<LAYOUT, kTile>(a, tiles, his, st);
+    return launch_index<LAYOUT, LAYOUT == EDPP_KO ? kTile : kPairTile>(a, tiles, stride, his, st);
+  if (a.buckets >= index_buckets<LAYOUT>())
+    return launch_index<LAYOUT, kTile>(a, tiles, stride, his, st);
   constexpr auto kernel = split_scatter_kernel<kScatterThreads, LAYOUT, kTile, false>;
   const int s = prepare_kernel<kernel>(
       kScatterThreads, scatter_smem_bytes<kScatterThreads, LAYOUT, kTile>(index_buckets<LAYOUT>(), true),
@@ -697,7 +719,7 @@ int launch_scatter(const SplitArgs &a, int64_t tiles, const int32_t *his, cudaSt
   if (s != EDPP_OK) return s;
   const bool bulk = bulk_runs<LAYOUT>(a);
   kernel<<<static_cast<unsigned>(tiles), kScatterThreads, scatter_smem_bytes<kScatterThreads, LAYOUT, kTile>(a.buckets, bulk),
-           st>>>(a.keys_in, a.keys_out, a.vals_in, a.vals_out, a.n, a.buckets, a.shift, tiles, his,
+           st>>>(a.keys_in, a.keys_out, a.vals_in, a.vals_out, a.n, a.buckets, a.shift, stride, his,
                  a.tma, bulk, kDefaultWaitNs, fault_word(), FusedArgs{});
   return launch_status();
 }
@@ -779,6 +801,10 @@ template <int LAYOUT> int split_fused(const SplitArgs &a, char *ws, cudaStream_t
   return EDPP_ENOMEM;
 }
 
+// Tiles from which a histogram block takes four: 8 blocks per SM are left then.
+constexpr int64_t kHistFour = 4 * 8 * kGb300Sms;
+constexpr int64_t round4(int64_t x) { return (x + 3) / 4 * 4; }
+
 template <int LAYOUT>
 int split_layout(const int32_t *keys_in, int32_t *keys_out, int32_t *bucket_start, int64_t n,
                  int buckets, const int32_t *vals_in, int32_t *vals_out, void *ws, size_t ws_bytes,
@@ -787,26 +813,31 @@ int split_layout(const int32_t *keys_in, int32_t *keys_out, int32_t *bucket_star
   const int tile = split_tile<LAYOUT>(buckets);
   const int64_t tiles = (n + tile - 1) / tile;
   int32_t *his = static_cast<int32_t *>(ws);
-  const int64_t hlen = tiles * buckets;
-  void *scan_ws = static_cast<char *>(ws) + his_bytes(tiles, buckets);
-  const size_t scan_ws_bytes = ws_bytes - his_bytes(tiles, buckets);
+  const bool four = tiles >= kHistFour && aligned16(ws);
+  const int64_t stride = four ? round4(tiles) : tiles;
+  const int64_t hlen = stride * buckets;
+  void *scan_ws = static_cast<char *>(ws) + his_bytes(stride, buckets);
+  const size_t scan_ws_bytes = ws_bytes - his_bytes(stride, buckets);
   const SplitArgs a{keys_in, keys_out, vals_in, vals_out, bucket_start, n, buckets, shift,
                     aligned16(keys_in) && (LAYOUT != EDPP_KVS_SOA || aligned16(vals_in)), exact};
   int s = split_fused<LAYOUT>(a, static_cast<char *>(ws), st);
   if (s != EDPP_ENOMEM) return s;
-  const auto hist = tile == kTile ? split_hist_kernel<LAYOUT, kTile> : split_hist_kernel<LAYOUT, kPairTile>;
-  hist<<<static_cast<unsigned>(tiles), kHistThreads, 0, st>>>(keys_in, n, buckets, shift, tiles, his,
-                                                              aligned16(keys_in));
+  const auto hist = four ? (tile == kTile ? split_hist_kernel<LAYOUT, kTile, 4>
+                                          : split_hist_kernel<LAYOUT, kPairTile, 4>)
+                         : (tile == kTile ? split_hist_kernel<LAYOUT, kTile, 1>
+                                          : split_hist_kernel<LAYOUT, kPairTile, 1>);
+  hist<<<static_cast<unsigned>(four ? stride / 4 : tiles), kHistThreads, 0, st>>>(
+      keys_in, n, buckets, shift, stride, his, aligned16(keys_in));
   s = launch_status();
   if (s != EDPP_OK) return s;
   s = edpp_scan_exclusive_i32(his, his, hlen, EDPP_SCAN_LOOKBACK, scan_ws, scan_ws_bytes, st);
   if (s != EDPP_OK) return s;
   if (bucket_start) {
-    bucket_start_kernel<<<(buckets + 255) / 256, 256, 0, st>>>(his, tiles, buckets, bucket_start);
+    bucket_start_kernel<<<(buckets + 255) / 256, 256, 0, st>>>(his, stride, buckets, bucket_start);
     s = launch_status();
     if (s != EDPP_OK) return s;
   }
-  return launch_scatter<LAYOUT>(a, tiles, his, st);
+  return launch_scatter<LAYOUT>(a, tiles, stride, his, st);
 }
 
 // From kLsdBuckets buckets on, a split is two stable passes through a
@@ -819,7 +850,7 @@ constexpr int kLsdBuckets = 2048;
 size_t split_pass_ws_bytes(int64_t n, int buckets) {
   // enough for every layout's tile
   const int64_t tile = buckets <= kPairTileBuckets ? kPairTile : kTile;
-  const int64_t tiles = (n + tile - 1) / tile;
+  const int64_t tiles = round4((n + tile - 1) / tile);
   return std::max(his_bytes(tiles, buckets) +
                       edpp_scan_workspace_size(tiles * buckets, EDPP_I32, EDPP_SCAN_LOOKBACK),
                   fused_ws_bytes(n, buckets));

@@ -53,3 +53,17 @@ def test_both_rankings(cuda, edpp, buckets, layout, exact):
             assert cuda.equal(k, wk) and cuda.equal(s, ws), n
             assert v is None or cuda.equal(v, wv), n
     assert edpp.sync_status() == edpp.EDPP_OK
+
+
+@pytest.mark.parametrize("layout,buckets", [("ko", 2), ("ko", 1024), ("soa", 64), ("soa", 256),
+                                            ("aos", 256)])
+def test_four_tiles_per_histogram_block(cuda, edpp, layout, buckets):
+    # from 4864 tiles on a histogram block counts four; rows padded to four tiles
+    tile = 6144 if layout != "ko" and buckets <= 64 else 8192
+    for n in (4864 * tile - tile, 4864 * tile, 4864 * tile + 1, 4866 * tile - 3):
+        vals = cuda.arange(n, device="cuda", dtype=cuda.int32)
+        keys = cuda.randint(-2**31, 2**31 - 1, (n,), device="cuda", dtype=cuda.int32)
+        wk, wv, ws = _want(cuda, keys, vals, buckets)
+        k, v, s = _split(edpp, cuda, keys, vals, buckets, layout, False)
+        assert cuda.equal(k, wk) and cuda.equal(s, ws), n
+        assert v is None or cuda.equal(v, wv), n
