@@ -37,6 +37,7 @@
 #include <algorithm>
 #include <mutex>
 
+#include "batch_plan.h"
 #include "scan_pipe.h"
 #include "scan_tile.cuh"
 
@@ -57,6 +58,7 @@ constexpr int kTileBytes = kScanThreads * kChunks * 16;
 constexpr int kStages = 12;      // 192 KB of tile buffers per block
 constexpr int kMaxBlocks = 256;  // words a prefix warp reads per wave: 8 per lane
 constexpr size_t kHeader = 256;
+constexpr uint32_t kFlagTail = kFlagIncl, kFlagHead = kFlagAgg;  // of a published tile sum
 static_assert(kStages % kReduceWarps == 0 && kStages % kGroups == 0,
               "a buffer always has the same reduce warp and scan group");
 
@@ -104,11 +106,57 @@ __device__ __forceinline__ void scan_group_sync(int group) {
   asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "n"(kScanThreads) : "memory");
 }
 
-template <typename T, bool kInclusive>
+// Where a tile lies.  head: its prefix starts from zero (kSegmented only).
+struct TileAt {
+  int64_t base;
+  int32_t count, head;
+};
+
+// One array cut into tiles.
+template <typename T> struct ArrayTiles {
+  static constexpr bool kSegmented = false;
+  int64_t n, num_tiles;
+  __device__ __forceinline__ TileAt at(int64_t tile) const {
+    constexpr int kTile = kTileBytes / sizeof(T);
+    return {tile * kTile, static_cast<int32_t>(min64(kTile, n - tile * kTile)), 0};
+  }
+};
+
+// The scan tiles of a batch: tile i is a task's tile of its segment, and every
+// segment's first tile is a head.  A task outside the plan's tables is recorded
+// and counts no elements.
+struct TaskTiles {
+  static constexpr bool kSegmented = true;
+  const DevSeg *segs;
+  const DevTask *tasks;
+  int num_segs;
+  int64_t num_tiles;
+  unsigned *fault;
+  __device__ __forceinline__ TileAt at(int64_t tile) const {
+    constexpr int kTile = kTileBytes / 4;
+    const DevTask t = tasks[tile];
+    bool ok = t.seg >= 0 && t.seg < num_segs;
+    DevSeg seg{};
+    if (ok) seg = segs[t.seg];
+    ok = ok && t.tile >= 0 && t.tile < seg.tiles;
+    if (!ok) raise_fault(fault, EDPP_FAULT_PLAN);
+    if (!ok) return {0, 0, 1};
+    const int64_t off = static_cast<int64_t>(t.tile) * kTile;
+    return {seg.off + off, static_cast<int32_t>(min64(kTile, seg.len - off)), t.tile == 0};
+  }
+};
+
+// Bit i set for the words i of this lane group that are at most `last`.
+__device__ __forceinline__ uint32_t up_to(int last) {
+  return last < 0 ? 0u : last >= 31 ? 0xffffffffu : (2u << last) - 1u;
+}
+
+template <typename T, bool kInclusive, typename Tiles>
 __global__ void __launch_bounds__(kThreads, 1)
-    scan_pipe_kernel(const T *in, T *out, int64_t n, int64_t num_tiles,
-                     LookbackState<T> st, unsigned *abort_flag, uint64_t timeout_ns,
-                     unsigned *fault) {
+    scan_pipe_kernel(const T *in, T *out, Tiles tiles, LookbackState<T> st, unsigned *abort_flag,
+                     uint64_t timeout_ns, unsigned *fault) {
+  constexpr bool kSegmented = Tiles::kSegmented;
+  const int64_t num_tiles = tiles.num_tiles;
   constexpr int E = Chunk<T>::E;
   constexpr int CH = kChunks, kTile = kTileBytes / sizeof(T), stages = kStages;
   using W = typename Wide<T>::type;
@@ -116,6 +164,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   __shared__ PipeShared sh;
   __shared__ T pre[2 * kStages];
   __shared__ W carry[kPrefixWarps];
+  __shared__ TileAt meta[kSegmented ? kStages : 1];  // of the tile in each buffer
   __shared__ T tot[kGroups][2][kScanWarps * CH];  // [group][alternating][row k][warp]
   const int lane = threadIdx.x & 31;
   // scan warps count within their group; the other roles follow the groups
@@ -147,9 +196,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     int s = group, p = group;  // ring positions of the tile and of its prefix
     uint32_t sp = 0, pp = 0, half = 0;
     for (int64_t i = group; i < steps; i += kGroups, half ^= 1u) {
-      const int64_t base = (i * G + b) * kTile;
-      const int count = static_cast<int>(min64(kTile, n - base));
       if (!dead) dead = !wait(&sh.full[s], sp);
+      const TileAt where = kSegmented ? meta[s] : tiles.at(i * G + b);
+      const int64_t base = where.base;
+      const int count = where.count;
       Chunk<T> c[CH];
       T incl[CH];
       const uint4 *src = reinterpret_cast<const uint4 *>(buf(s)) + tid;
@@ -247,6 +297,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     for (int64_t i = warp - kScanWarps; i < steps; i += kReduceWarps) {
       const int s = static_cast<int>(i % stages);
       if (!wait(&sh.full[s], static_cast<uint32_t>(i / stages) & 1u)) break;
+      const uint32_t flag = kSegmented && meta[s].head ? kFlagHead : kFlagTail;
       const uint4 *src = reinterpret_cast<const uint4 *>(buf(s)) + lane;
       // eight chains of additions, joined pairwise
       T acc[8];
@@ -271,24 +322,36 @@ __global__ void __launch_bounds__(kThreads, 1)
       __syncwarp();
       if (lane == 0) mbar_arrive(&sh.empty[s]);
       const T v = warp_sum(acc[0]);
-      if (lane == 0) st.publish(i * G + b, kFlagIncl, v);
+      if (lane == 0) st.publish(i * G + b, flag, v);
     }
   } else if (warp == kScanWarps + kReduceWarps) {
     // ---- load ----
     int64_t i = 0;
+    TileAt ahead{};  // kSegmented: lane l looks up step l of the next 32
     for (; i < steps; ++i) {
       const int s = static_cast<int>(i % stages);
+      if (kSegmented && (i & 31) == 0 && i + lane < steps) ahead = tiles.at((i + lane) * G + b);
+      TileAt where;
+      if (kSegmented) {
+        where.base = __shfl_sync(0xffffffffu, ahead.base, static_cast<int>(i & 31));
+        where.count = __shfl_sync(0xffffffffu, ahead.count, static_cast<int>(i & 31));
+        where.head = __shfl_sync(0xffffffffu, ahead.head, static_cast<int>(i & 31));
+      } else {
+        where = tiles.at(i * G + b);
+      }
       if (i >= stages && !wait(&sh.empty[s], static_cast<uint32_t>(i / stages - 1) & 1u)) break;
-      const int64_t base = (i * G + b) * kTile;
-      const int count = static_cast<int>(min64(kTile, n - base));
+      const int64_t base = where.base;
+      const int count = where.count;
       const uint32_t bytes = (static_cast<uint32_t>(count) * sizeof(T)) & ~15u;
-      if (count < kTile) {  // the last tile: the rest by plain accesses, zeros past the end
+      if (count < kTile) {  // a last tile: the rest by plain accesses, zeros past the end
         T *dst = buf(s);
         for (int j = static_cast<int>(bytes / sizeof(T)) + lane; j < kTile; j += 32)
           dst[j] = j < count ? in[base + j] : zero_of<T>();
+        fence_proxy_async_smem();  // before a later bulk copy into the same bytes
         __syncwarp();
       }
       if (lane == 0) {
+        if (kSegmented) meta[s] = where;
         mbar_arrive_expect_tx(&sh.full[s], bytes);
         if (bytes) tma_load_1d(buf(s), in + base, bytes, &sh.full[s]);
       }
@@ -309,6 +372,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       constexpr int kPer = kMaxBlocks / 32;
       T v[kPer];
       uint32_t have = 0;  // bit j: word lane + 32 j has been read
+      uint32_t heads = 0;  // kSegmented, bit j: it is a head's
 #pragma unroll
       for (int j = 0; j < kPer; ++j) {
         v[j] = zero_of<T>();
@@ -322,7 +386,8 @@ __global__ void __launch_bounds__(kThreads, 1)
           if (!((have >> j) & 1u)) {
             uint32_t f;
             st.read(first + lane + 32 * j, f, v[j]);
-            if (f == kFlagIncl) have |= 1u << j;
+            if (f != kFlagNone) have |= 1u << j;
+            if (kSegmented && f == kFlagHead) heads |= 1u << j;
           }
         if (__all_sync(0xffffffffu, have == (1u << kPer) - 1u)) break;
         if (t0 == 0) t0 = globaltimer_ns();
@@ -338,11 +403,24 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
       }
       if (!ok) break;
+      // kSegmented: sums start at the last head up to this tile (`from`) and of
+      // the wave (`last`); without one (-1), the carry comes in too
+      int from = -1, last = -1;
+      if (kSegmented) {
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+          const uint32_t m = __ballot_sync(0xffffffffu, (heads >> j) & 1u);
+          const uint32_t mb = m & up_to(static_cast<int>(b) - 32 * j);
+          if (m) last = 32 * j + 31 - __clz(m);
+          if (mb) from = 32 * j + 31 - __clz(mb);
+        }
+      }
       T before = zero_of<T>(), total = zero_of<T>();
 #pragma unroll
       for (int j = 0; j < kPer; ++j) {
-        total = op_add(total, v[j]);
-        if (lane + 32 * j < b) before = op_add(before, v[j]);
+        const int at = lane + 32 * j;
+        if (at >= last) total = op_add(total, v[j]);
+        if (at >= from && at < b) before = op_add(before, v[j]);
       }
       before = warp_sum(before);
       total = warp_sum(total);
@@ -354,10 +432,10 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
       if (lane == 0) {
         const int nq = q + 1 == kPrefixWarps ? 0 : q + 1;
-        carry[nq] = op_add(sum, W(total));
+        carry[nq] = op_add(last < 0 ? sum : W(0), W(total));
         mbar_arrive(&sh.carried[nq]);
         const int p = static_cast<int>(i % (2 * stages));
-        pre[p] = static_cast<T>(op_add(sum, W(before)));
+        pre[p] = static_cast<T>(op_add(from < 0 ? sum : W(0), W(before)));
         mbar_arrive(&sh.ready[p]);
       }
       __syncwarp();
@@ -365,18 +443,35 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
 }
 
-template <typename T, bool kInclusive>
-int launch_pipe(const T *in, T *out, int64_t n, char *header, cudaStream_t st, uint64_t timeout_ns,
-                unsigned *fault) {
-  constexpr int64_t kTile = kTileBytes / sizeof(T);
+// One cooperative launch over `tiles`, its state words zeroed by the caller.
+template <typename T, bool kInclusive, typename Tiles>
+int launch_pipe(const T *in, T *out, Tiles tiles, void *words, unsigned *abort_flag,
+                cudaStream_t st, uint64_t timeout_ns, unsigned *fault) {
   constexpr int kSmem = kStages * kTileBytes;
-  auto *kernel = scan_pipe_kernel<T, kInclusive>;
+  auto *kernel = scan_pipe_kernel<T, kInclusive, Tiles>;
+  LookbackState<T> state;
+  state.bind(words, tiles.num_tiles);
+  const int64_t blocks = std::min<int64_t>({tiles.num_tiles, device_sm_count(), kMaxBlocks});
+  void *args[] = {&in, &out, &tiles, &state, &abort_flag, &timeout_ns, &fault};
+  if (cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(kernel),
+                                  dim3(static_cast<unsigned>(blocks)), dim3(kThreads), args, kSmem,
+                                  st) != cudaSuccess) {
+    cudaGetLastError();  // not co-resident: the caller takes another form
+    return EDPP_ENOMEM;
+  }
+  return launch_status();
+}
+
+// Whether a block of the kernel fits an SM of this device (checked once).
+template <typename T, bool kInclusive, typename Tiles> bool pipe_fits() {
+  constexpr int kSmem = kStages * kTileBytes;
   static std::once_flag once[64];
   static bool fits[64];
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) dev = 0;
-  std::call_once(once[dev], [dev, kernel] {
+  std::call_once(once[dev], [dev] {
+    auto *kernel = scan_pipe_kernel<T, kInclusive, Tiles>;
     int per_sm = 0;
     fits[dev] = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) ==
                     cudaSuccess &&
@@ -385,23 +480,7 @@ int launch_pipe(const T *in, T *out, int64_t n, char *header, cudaStream_t st, u
                 per_sm > 0;
     if (!fits[dev]) cudaGetLastError();
   });
-  if (!fits[dev]) return EDPP_ENOMEM;
-  int64_t tiles = (n + kTile - 1) / kTile;
-  const int64_t blocks = std::min<int64_t>({tiles, device_sm_count(), kMaxBlocks});
-  if (cudaMemsetAsync(header, 0, kHeader + LookbackState<T>::bytes(tiles), st) != cudaSuccess)
-    return EDPP_ECUDA;
-  LookbackState<T> state;
-  state.bind(header + kHeader, tiles);
-  unsigned *abort_flag = reinterpret_cast<unsigned *>(header + 8);
-  void *args[] = {const_cast<T **>(&in), &out, &n, &tiles, &state, &abort_flag,
-                  &timeout_ns, &fault};
-  if (cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(kernel),
-                                  dim3(static_cast<unsigned>(blocks)), dim3(kThreads), args, kSmem,
-                                  st) != cudaSuccess) {
-    cudaGetLastError();  // not co-resident: the caller takes another form
-    return EDPP_ENOMEM;
-  }
-  return launch_status();
+  return fits[dev];
 }
 
 }  // namespace
@@ -414,7 +493,23 @@ template <typename T> size_t scan_pipe_state_bytes(int64_t n) {
 template <typename T, bool kInclusive>
 int scan_pipe(const T *in, T *out, int64_t n, char *header, cudaStream_t st, uint64_t timeout_ns,
               unsigned *fault) {
-  return launch_pipe<T, kInclusive>(in, out, n, header, st, timeout_ns, fault);
+  if (!pipe_fits<T, kInclusive, ArrayTiles<T>>()) return EDPP_ENOMEM;
+  constexpr int64_t kTile = kTileBytes / sizeof(T);
+  const ArrayTiles<T> tiles{n, (n + kTile - 1) / kTile};
+  if (cudaMemsetAsync(header, 0, kHeader + LookbackState<T>::bytes(tiles.num_tiles), st) !=
+      cudaSuccess)
+    return EDPP_ECUDA;
+  return launch_pipe<T, kInclusive>(in, out, tiles, header + kHeader,
+                                    reinterpret_cast<unsigned *>(header + 8), st, timeout_ns,
+                                    fault);
+}
+
+int scan_pipe_tasks(const int32_t *in, int32_t *out, const DevSeg *segs, const DevTask *tasks,
+                    int num_segs, int64_t num_tiles, void *words, unsigned *abort_flag,
+                    cudaStream_t st, uint64_t timeout_ns, unsigned *fault) {
+  if (!pipe_fits<int32_t, false, TaskTiles>()) return EDPP_ENOMEM;
+  return launch_pipe<int32_t, false>(in, out, TaskTiles{segs, tasks, num_segs, num_tiles, fault},
+                                     words, abort_flag, st, timeout_ns, fault);
 }
 
 #define EDPP_PIPE(T)                                                                             \

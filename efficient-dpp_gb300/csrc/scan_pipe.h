@@ -20,4 +20,15 @@ template <typename T, bool kInclusive>
 int scan_pipe(const T *in, T *out, int64_t n, char *header, cudaStream_t st, uint64_t timeout_ns,
               unsigned *fault);
 
+struct DevSeg;
+struct DevTask;
+
+// Exclusive scan of every segment of a batch (batch_plan.h): `tasks` are the
+// scan tiles, each segment's in order from tile 0.  Segment offsets multiples of
+// 4 elements, in and out 16-byte aligned.  `words`: num_tiles zeroed 8-byte
+// words.  EDPP_ENOMEM as above.
+int scan_pipe_tasks(const int32_t *in, int32_t *out, const DevSeg *segs, const DevTask *tasks,
+                    int num_segs, int64_t num_tiles, void *words, unsigned *abort_flag,
+                    cudaStream_t st, uint64_t timeout_ns, unsigned *fault);
+
 }  // namespace edpp
