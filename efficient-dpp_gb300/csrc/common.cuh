@@ -175,6 +175,11 @@ __device__ __forceinline__ uint4 ld_v4_policy(const uint4 *p, uint64_t policy) {
   return v;
 }
 
+// Brings [p, p + bytes) into L2 (16-byte aligned, a multiple of 16).
+__device__ __forceinline__ void l2_prefetch(const void *p, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+
 // Bulk copy shared -> global (bulk-group completion).
 __device__ __forceinline__ void tma_store_1d(void *gmem_dst, const void *smem_src, uint32_t bytes) {
   asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(gmem_dst),

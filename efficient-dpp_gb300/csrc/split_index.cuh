@@ -75,6 +75,12 @@ __global__ void __launch_bounds__(kIndexThreads, index_blocks<LAYOUT, TILE, kFus
       if (LAYOUT == EDPP_KVS_SOA) tma_load_1d(s_vals, vals_in + base, bulk_elems * 4, &bar);
     }
   }
+  // As in split_scatter_kernel; pairs in one array gain 1-2% (2^28, 8 / 256
+  // buckets 1.288 / 1.338 -> 1.271 / 1.314 ms), the other layouts nothing.
+  const int64_t ahead = base + static_cast<int64_t>(kGb300Sms) * TILE;
+  if (!kFused && LAYOUT == EDPP_KVS_AOS && tid == 32 && tma && ahead + TILE <= n) {
+    l2_prefetch(keys_in + 2 * ahead, TILE * 8);
+  }
   for (int i = static_cast<int>(bulk_elems) + tid; i < count; i += THREADS) {
     if (LAYOUT == EDPP_KVS_AOS) {
       s_pairs[i] = make_int2(keys_in[2 * (base + i)], keys_in[2 * (base + i) + 1]);
