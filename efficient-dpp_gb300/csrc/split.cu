@@ -800,6 +800,7 @@ size_t fused_ws_bytes(int64_t n, int buckets) {
 }
 
 template <int LAYOUT> int split_fused(const SplitArgs &a, char *ws, cudaStream_t st) {
+  if (!aligned16(ws)) return EDPP_ENOMEM;  // his is read in 16-byte quads
   const int64_t sms = device_sm_count();
   auto fits = [&](int64_t tile, int64_t blocks) {
     const int64_t tiles = (a.n + tile - 1) / tile;

@@ -91,3 +91,16 @@ def test_captured_and_on_two_streams(cuda, edpp):
     cuda.cuda.synchronize()
     assert all(cuda.equal(o[0], wk) and cuda.equal(o[1], wv) for o in outs)
     assert edpp.sync_status() == edpp.EDPP_OK
+
+
+@pytest.mark.parametrize("n", [50_021, 3_000_001, 4864 * 8192 + 5])
+def test_workspace_off_16_bytes(cuda, edpp, n):
+    # a workspace 8 bytes past a 16-byte boundary: neither the one-launch form
+    # nor the four-tile histogram reads or writes it in 16-byte words
+    keys = cuda.randint(0, 2**31 - 1, (n,), device="cuda", dtype=cuda.int32)
+    vals = cuda.arange(n, device="cuda", dtype=cuda.int32)
+    wk, wv, s = _want(cuda, keys, vals, 256)
+    ws = edpp.workspace(edpp.split_workspace_bytes(n, 256, "soa") + 8)[8:]
+    k, v, st = edpp.split(keys, 256, values=vals, bucket_start=True, ws=ws)
+    assert cuda.equal(k, wk) and cuda.equal(v, wv) and cuda.equal(st, s)
+    assert edpp.sync_status() == edpp.EDPP_OK
