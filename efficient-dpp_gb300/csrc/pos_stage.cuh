@@ -43,6 +43,30 @@ template <int NT, int TILE> struct PosStage {
       const int pos = position(it);
       br[it] = pos < count ? static_cast<uint32_t>(bucket_at(pos)) : 0u;
     }
+    // Keys already in bucket order put a whole warp on one counter, 32 atomics
+    // in a row: where a warp's first and last element share a bucket, a step of
+    // one bucket takes one atomic (split of 2^27 sorted pairs, 256 / 512 buckets
+    // 0.885 / 0.969 -> 0.582 / 0.647 ms; uniform keys 0 to 1% slower for the test).
+    const int lane = threadIdx.x & 31;
+    const int first = position(0) - lane, last = min(first + kSeg, count) - 1;
+    if (last >= first && bucket_at(first) == bucket_at(last)) {
+      const uint32_t b = static_cast<uint32_t>(bucket_at(first)), shb = (b & 1u) * 16u;
+#pragma unroll
+      for (int it = 0; it < kIters; ++it) {
+        const bool valid = position(it) < count;
+        const unsigned mine = __ballot_sync(0xffffffffu, valid && br[it] == b);
+        if (mine == 0xffffffffu) {
+          uint32_t old = 0;
+          if (lane == 0) old = atomicAdd(&words[b >> 1], 32u << shb);
+          old = (__shfl_sync(0xffffffffu, old, 0) >> shb) & 0xffffu;
+          br[it] |= (old + lane) << 16;
+        } else if (valid) {
+          const uint32_t sh = (br[it] & 1u) * 16u;
+          br[it] |= ((atomicAdd(&words[br[it] >> 1], 1u << sh) >> sh) & 0xffffu) << 16;
+        }
+      }
+      return;
+    }
 #pragma unroll
     for (int it = 0; it < kIters; ++it) {
       const uint32_t sh = (br[it] & 1u) * 16u;

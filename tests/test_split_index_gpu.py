@@ -47,7 +47,11 @@ def test_both_rankings(cuda, edpp, buckets, layout, exact):
         uniform = cuda.randint(-2**31, 2**31 - 1, (n,), generator=g, device="cuda", dtype=cuda.int32)
         one = uniform & ~(buckets - 1) | (buckets - 1)
         skew = cuda.where(uniform > 0, one, uniform)
-        for keys in (uniform, one, skew):
+        ordered = cuda.sort(uniform & (buckets - 1))[0]
+        ends = uniform.clone()  # a warp's first and last element share a bucket
+        ends[::128] = 5
+        ends[127::128] = 5
+        for keys in (uniform, one, skew, ordered, ends):
             wk, wv, ws = _want(cuda, keys, vals, buckets)
             k, v, s = _split(edpp, cuda, keys, vals, buckets, layout, exact)
             assert cuda.equal(k, wk) and cuda.equal(s, ws), n
