@@ -90,8 +90,8 @@ def call_launches(name, p, method="tiled"):
     """Kernels of this library one call launches."""
     if name not in ("gather", "scatter"):
         return 1
-    if method == "tiled":  # count, scan, partition, refine, (fetch, refine,) apply
-        return 7 if name == "gather" else 5
+    if method == "tiled":  # group, fetch, restore; count, scan, partition, refine, apply
+        return 3 if name == "gather" else 5
     if method == "sweep" or p == 1:
         return p
     return 5 if name == "gather" else 4  # count, bases, partition, (fetch,) apply

@@ -646,7 +646,12 @@ __global__ void __launch_bounds__(kThreads, 4)
 // ---- host planner --------------------------------------------------------------
 namespace {
 
-constexpr int64_t kPipeTiles = 8 * kGb300Sms;  // scan tiles from which the pipelined scan runs
+// Scan tiles from which the pipelined scan runs.  It costs some 6 us more to
+// launch (cooperatively, after the kernels before it have drained) and 2.5 ns
+// less per tile: batches of 512 segments, 1.7e7 elements (1360 scan tiles) 92 us
+// without and 97 with it, 6.7e7 elements (5400) 257 and 246; 4096 segments of
+// 6.7e7 elements even, of 2.7e8 881 and 847.
+constexpr int64_t kPipeTiles = 4096;
 constexpr size_t kHdrB = 256;  // ticket (u64) + abort flag (u32)
 
 int build_plan(const edpp_segment *in, int num, const edpp_batch_tuning *tune, BatchPlanImpl &p) {
@@ -848,8 +853,7 @@ int edpp_batch_launch(const edpp_batch_plan *plan, const int32_t *in0, const int
                   p.num_segs};
   if (p.schedule == EDPP_BATCH_SCHEDULE_KINDS) {
     // Many scan tiles: the pipelined scan (scan_pipe.cu).  4096 segments all
-    // scan, 2^30 elements: 2.00 -> 1.45 ms; its cooperative launch costs some 3 us,
-    // so small batches keep one block per tile.
+    // scan, 2^30 elements: 2.00 -> 1.31 ms.
     bool scanned = p.n_scan == 0;
     if (!scanned && p.n_scan >= kPipeTiles && p.scan_aligned && aligned16(in0) && aligned16(out0)) {
       const int s = scan_pipe_tasks(in0, out0, dsegs, dtasks, p.num_segs, p.n_scan, w + p.off_state,

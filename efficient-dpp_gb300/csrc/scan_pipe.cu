@@ -327,10 +327,19 @@ __global__ void __launch_bounds__(kThreads, 1)
   } else if (warp == kScanWarps + kReduceWarps) {
     // ---- load ----
     int64_t i = 0;
-    TileAt ahead{};  // kSegmented: lane l looks up step l of the next 32
+    // kSegmented: lane l looks up step l of the next 32, with the elements past
+    // the tile's last whole 16 bytes, so that no step waits for them
+    TileAt ahead{};
+    T rest[E - 1];
     for (; i < steps; ++i) {
       const int s = static_cast<int>(i % stages);
-      if (kSegmented && (i & 31) == 0 && i + lane < steps) ahead = tiles.at((i + lane) * G + b);
+      if (kSegmented && (i & 31) == 0 && i + lane < steps) {
+        ahead = tiles.at((i + lane) * G + b);
+        const int rem = ahead.count % E;
+#pragma unroll
+        for (int e = 0; e < E - 1; ++e)
+          rest[e] = e < rem ? in[ahead.base + ahead.count - rem + e] : zero_of<T>();
+      }
       TileAt where;
       if (kSegmented) {
         where.base = __shfl_sync(0xffffffffu, ahead.base, static_cast<int>(i & 31));
@@ -344,9 +353,20 @@ __global__ void __launch_bounds__(kThreads, 1)
       const int count = where.count;
       const uint32_t bytes = (static_cast<uint32_t>(count) * sizeof(T)) & ~15u;
       if (count < kTile) {  // a last tile: the rest by plain accesses, zeros past the end
-        T *dst = buf(s);
-        for (int j = static_cast<int>(bytes / sizeof(T)) + lane; j < kTile; j += 32)
-          dst[j] = j < count ? in[base + j] : zero_of<T>();
+        const int whole = count - count % E;
+        T v = zero_of<T>();
+        if (kSegmented) {
+#pragma unroll
+          for (int e = 0; e < E - 1; ++e) {
+            const T y = shfl_idx(rest[e], static_cast<int>(i & 31));
+            if (lane == e) v = y;
+          }
+        } else if (whole + lane < count) {
+          v = in[base + whole + lane];
+        }
+        if (lane < E) buf(s)[whole + lane] = v;
+        uint4 *chunks = reinterpret_cast<uint4 *>(buf(s));
+        for (int c = whole / E + 1 + lane; c < kTile / E; c += 32) chunks[c] = make_uint4(0, 0, 0, 0);
         fence_proxy_async_smem();  // before a later bulk copy into the same bytes
         __syncwarp();
       }

@@ -1,5 +1,5 @@
 """Batched scans above and below the tile count that takes the pipelined scan
-(1216 tiles of 4096): segments of one element, of one tile, ragged and long
+(4096 tiles of 4096 elements): segments of one element, of one tile, ragged and long
 ones, so that heads fall everywhere in a wave; unaligned offsets keep the
 tile-per-block kernel; graph replay."""
 import numpy as np
@@ -7,7 +7,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-PIPE_TILES = 1216
+PIPE_TILES = 4096
 
 
 def _lengths(kind, tiles):
@@ -35,7 +35,7 @@ def _want(cuda, segs, x):
 
 
 @pytest.mark.parametrize("shift", [0, 1])
-@pytest.mark.parametrize("tiles", [PIPE_TILES - 1, PIPE_TILES, 5000])
+@pytest.mark.parametrize("tiles", [PIPE_TILES - 1, PIPE_TILES, 9001])
 @pytest.mark.parametrize("kind", ["short", "mixed", "long"])
 def test_scan_segments(cuda, edpp, kind, tiles, shift):
     from edpp import batch
