@@ -12,9 +12,10 @@
 //            is scanned; same ranking as split.cu, 64-bucket-class tiles
 //
 // Two schedules (edpp_batch_tuning.schedule):
-//   KINDS  one launch per kind, one block per tile: scan tiles, gather tiles,
-//          HIST tiles, one block per split segment scanning its histogram,
-//          SPLIT tiles.  Stream order separates the kinds; a scan tile waits
+//   KINDS  one launch per kind, one block per tile: scan tiles (many of them
+//          through the pipelined scan of scan_pipe.cu), gather tiles, HIST
+//          tiles, one block per split segment scanning its histogram, SPLIT
+//          tiles.  Stream order separates the kinds; a scan tile waits
 //          only on lower tiles of its segment (lower block indices).
 //   QUEUE  one persistent kernel; blocks take tasks from one atomic ticket in
 //          queue order.  The block that finishes a segment's last HIST tile

@@ -194,7 +194,7 @@ __device__ __forceinline__ void flush_runs(const int2 (&pr)[PER], const int (&w)
   }
 }
 
-// The pipelined stages (partition, refine, fetch) group a tile with four
+// The pipelined stages (partition, refine) group a tile with four
 // barriers: (A) rank atomics done; claim_runs; (B) staging offsets known;
 // staging writes and publish_run_bases; (C) runs staged; read-out.
 //
@@ -1077,7 +1077,7 @@ int ensure_win_attrs() {
   return st[dev];
 }
 
-// pairs_a: 8-byte pairs {x, y} (partition and fetch output); pairs_b: the
+// pairs_a: 8-byte pairs {x, y} (the partition's output); pairs_b: the
 // refine's output as 16-bit window offsets (at pairs_b) and 32-bit values
 // (at pairs_b + soa_val), both 16-byte aligned.
 struct TLayout {

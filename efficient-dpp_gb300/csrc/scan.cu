@@ -2,10 +2,10 @@
 //
 // Three schemes, all producing the same integer results:
 //
-//  LOOKBACK  one launch, one tile per block, tiles taken from an atomic
-//            ticket so progress never depends on launch order; a tile's
-//            exclusive prefix comes from a decoupled look-back over the
-//            published aggregates of its predecessors (bounded waits).
+//  LOOKBACK  one launch that publishes every tile's aggregate and adds up those
+//            before it (bounded waits): large aligned arrays by the pipelined
+//            kernel of scan_pipe.cu, small ones in one thread-block cluster,
+//            the rest one tile per block with a decoupled look-back.
 //            Traffic 2n: each element read once and written once.  Stands
 //            in for the reference's chained scan with adjacent
 //            synchronisation (opencl/primitives/scanImpl.cpp:15-66,
@@ -16,8 +16,8 @@
 //            memory (scan_pipe.cu) or in L2 (rts_fused, rts_chunked) between
 //            its two reads: traffic 2n; where no cooperative grid fits, three
 //            launches (per-block reduction, scan of the block sums in one
-//            block, per-block rescan with the offset): traffic 3n.  The reference's RSS scan
-//            (opencl/primitives/scanImpl.cpp:69-160,
+//            block, per-block rescan with the offset): traffic 3n.  The
+//            reference's RSS scan (opencl/primitives/scanImpl.cpp:69-160,
 //            opencl/kernels/scan_global_RSS_kernel.cl:142-240) and
 //            scan_RTS_omp (openmp/test_scan_CPU.cpp:125-163).
 //  SSA       scan-then-propagate ("scan-scan-add"): per-block scans written
