@@ -11,6 +11,7 @@
 // device by edpp_autotune_plain and recorded.
 #include <dlfcn.h>
 
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -30,6 +31,7 @@ namespace {
 struct Entry {
   int prim, elem, cls, variant;
   float ms;
+  bool set;  // by edpp_tune_set, not by a file or the autotuner
 };
 
 const char *const kNames[] = {"scan_lookback", "scan_rts", "gather"};
@@ -38,6 +40,7 @@ constexpr int kPrims = 3;
 std::mutex g_mu;
 std::vector<Entry> g_table;
 bool g_loaded = false;
+std::atomic<bool> g_any_set{false};  // an entry of g_table has `set`
 
 int prim_of(const char *name) {
   for (int p = 0; p < kPrims; ++p)
@@ -75,18 +78,21 @@ std::string default_path() {
   return pkg + "/tuning/plain_gb300.tsv";
 }
 
-void set_locked(int prim, int elem, int cls, int variant, float ms) {
+void set_locked(int prim, int elem, int cls, int variant, float ms, bool set) {
+  if (set) g_any_set = true;
   for (Entry &e : g_table)
     if (e.prim == prim && e.elem == elem && e.cls == cls) {
       e.variant = variant;
       e.ms = ms;
+      e.set = set;
       return;
     }
-  g_table.push_back({prim, elem, cls, variant, ms});
+  g_table.push_back({prim, elem, cls, variant, ms, set});
 }
 
 int load_locked(const std::string &path) {
   g_table.clear();
+  g_any_set = false;
   g_loaded = true;
   if (path.empty()) return EDPP_OK;
   FILE *f = std::fopen(path.c_str(), "r");
@@ -107,7 +113,7 @@ int load_locked(const std::string &path) {
       status = EDPP_EINVAL;  // a malformed line is skipped and reported
       continue;
     }
-    set_locked(prim, elem, cls, variant, got >= 5 ? ms : 0.0f);
+    set_locked(prim, elem, cls, variant, got >= 5 ? ms : 0.0f, false);
   }
   std::fclose(f);
   return status;
@@ -117,10 +123,7 @@ void ensure_loaded_locked() {
   if (!g_loaded) load_locked(default_path());
 }
 
-}  // namespace
-
-int tuned_variant(int prim, int elem_bytes, int64_t length, int fallback) {
-  std::lock_guard<std::mutex> lk(g_mu);
+const Entry *nearest_locked(int prim, int elem_bytes, int64_t length) {
   ensure_loaded_locked();
   const int cls = class_of(length);
   const Entry *best = nullptr;
@@ -130,7 +133,22 @@ int tuned_variant(int prim, int elem_bytes, int64_t length, int fallback) {
         (std::abs(e.cls - cls) == std::abs(best->cls - cls) && e.cls > best->cls))
       best = &e;
   }
-  return best ? best->variant : fallback;
+  return best;
+}
+
+}  // namespace
+
+int tuned_variant(int prim, int elem_bytes, int64_t length, int fallback) {
+  std::lock_guard<std::mutex> lk(g_mu);
+  const Entry *e = nearest_locked(prim, elem_bytes, length);
+  return e ? e->variant : fallback;
+}
+
+int chosen_variant(int prim, int elem_bytes, int64_t length) {
+  if (!g_any_set.load(std::memory_order_acquire)) return -1;
+  std::lock_guard<std::mutex> lk(g_mu);
+  const Entry *e = nearest_locked(prim, elem_bytes, length);
+  return e && e->set ? e->variant : -1;
 }
 
 }  // namespace edpp
@@ -146,7 +164,7 @@ int edpp_tune_set(int primitive, int elem_bytes, int log2_length, int variant, f
     return EDPP_EINVAL;
   std::lock_guard<std::mutex> lk(edpp::g_mu);
   edpp::ensure_loaded_locked();
-  edpp::set_locked(primitive, elem_bytes, log2_length, variant, ms);
+  edpp::set_locked(primitive, elem_bytes, log2_length, variant, ms, true);
   return EDPP_OK;
 }
 
@@ -186,6 +204,7 @@ int edpp_tune_save(const char *path) {
 void edpp_tune_clear(void) {
   std::lock_guard<std::mutex> lk(edpp::g_mu);
   edpp::g_table.clear();
+  edpp::g_any_set = false;
   edpp::g_loaded = true;
 }
 
@@ -260,7 +279,10 @@ int edpp_autotune_plain(int primitive, const void *in, void *out, const int32_t 
   }
   *best_variant = best;
   if (best_ms) *best_ms = best_t;
-  return edpp_tune_set(primitive, elem_bytes, edpp::class_of(length), best, best_t);
+  std::lock_guard<std::mutex> lk(edpp::g_mu);
+  edpp::ensure_loaded_locked();
+  edpp::set_locked(primitive, elem_bytes, edpp::class_of(length), best, best_t, false);
+  return EDPP_OK;
 }
 
 }  // extern "C"

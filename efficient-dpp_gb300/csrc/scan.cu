@@ -769,6 +769,9 @@ int scan_impl(const T *in, T *out, int64_t n, int algo, void *ws, size_t ws_byte
   char *w = static_cast<char *>(ws);
 
   if (variant < 0 && algo != EDPP_SCAN_SSA && n <= small_max<T>())
+    variant = chosen_variant(
+        algo == EDPP_SCAN_LOOKBACK ? EDPP_TUNE_SCAN_LOOKBACK : EDPP_TUNE_SCAN_RTS, sizeof(T), n);
+  if (variant < 0 && algo != EDPP_SCAN_SSA && n <= small_max<T>())
     return launch_small<T, kInclusive>(in, out, n, st);
   if (algo == EDPP_SCAN_LOOKBACK) {
     if (variant < 0) variant = tuned_variant(EDPP_TUNE_SCAN_LOOKBACK, sizeof(T), n, 0);

@@ -16,6 +16,10 @@ namespace edpp {
 // class recorded for that primitive and element size, else `fallback`.
 int tuned_variant(int prim, int elem_bytes, int64_t length, int fallback);
 
+// The variant of that entry if edpp_tune_set recorded it, else -1: a choice
+// that goes before the rules by which a scan of moderate size leaves the table.
+int chosen_variant(int prim, int elem_bytes, int64_t length);
+
 // Scan of `length` elements of `elem_bytes` bytes (4: int32, 8: int64) with
 // an explicit variant of `algo` (EDPP_SCAN_LOOKBACK: tile shape, EDPP_SCAN_RTS:
 // slice length of the chunked form), for the autotuner.  Same arguments and
