@@ -4,8 +4,10 @@
 //
 //  LOOKBACK  one launch that publishes every tile's aggregate and adds up those
 //            before it (bounded waits): large aligned arrays by the pipelined
-//            kernel of scan_pipe.cu, small ones in one thread-block cluster,
-//            the rest one tile per block with a decoupled look-back.
+//            kernel of scan_pipe.cu, unaligned ones one tile per block with a
+//            decoupled look-back.  Where the array stays in L2 this scheme and
+//            RTS both run in two launches that wait for nothing, and in one
+//            thread-block cluster when small.
 //            Traffic 2n: each element read once and written once.  Stands
 //            in for the reference's chained scan with adjacent
 //            synchronisation (opencl/primitives/scanImpl.cpp:15-66,
@@ -29,6 +31,7 @@
 // the tile layout.
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 
 #include "scan_pipe.h"
 #include "scan_tile.cuh"
@@ -225,6 +228,166 @@ template <typename T, bool kInclusive>
 int launch_small(const T *in, T *out, int64_t n, cudaStream_t st) {
   return n <= kSmallBlocks * TSS<T, 4>::kTile ? launch_small_as<T, kInclusive, 4>(in, out, n, st)
                                               : launch_small_as<T, kInclusive, 8>(in, out, n, st);
+}
+
+// ---- middle sizes: two launches, one tile per block ----------------------------
+// scan_sums adds up every tile; scan_tiles scans them, each block adding up the
+// sums before its own tile.  Nothing waits inside a kernel, so there is no state
+// to zero and no cooperative launch, and the second launch is programmatic: its
+// blocks load and scan their tiles while the first kernel ends, and wait for its
+// sums only then.  The second read of the input comes from L2.  Bound by launch and
+// load latency up to a million elements, then by the input's read from DRAM and
+// again from L2 (2^23 int32: 4.0 TB/s of input and output).  Device time of one call
+// among others, us, against the pipelined, look-back and fused forms it took over
+// from (look-back / reduce-then-scan): int32 140000 elements 8.0 / 8.6 -> 3.6, 2^20
+// 11.6 / 12.3 -> 4.9, 2^22 13.2 / 16.9 -> 9.7, 2^23 22.8 / 23.3 -> 16.8; int64 2^20
+// 11.5 / 14.4 -> 7.4, 2^22 24.1 / 26.4 -> 22.8.
+//
+// 32 KB tiles.  256 threads x 8 chunks against 512 x 4: int32 2^22 9.7 and 10.9 us,
+// int64 140000 elements 7.4 and 5.2 us (64 KB tiles 8.2), so each has its own.
+template <typename T> struct TwoShape {
+  static constexpr int kThreads = sizeof(T) == 4 ? 256 : 512;
+  static constexpr int kChunks = sizeof(T) == 4 ? 8 : 4;
+  static constexpr int kBlocks = sizeof(T) == 4 ? 4 : 2;  // per SM
+  static constexpr int kWarps = kThreads / 32;
+  using S = TileScan<T, kThreads, kChunks>;
+};
+
+// The sum of float tiles: the float sum and the rounding errors left out of it.
+// (As doubles the sums bound the second kernel: 2^22 11.1 us, in pairs 9.7.)  Error
+// against 64 bits at 2^22: 1.8e-7 with the look-back's float sums, now 5.9e-8.
+struct FloatPair {
+  float hi, lo;
+  FloatPair() = default;
+  __device__ __forceinline__ explicit FloatPair(float x, float y = 0.f) : hi(x), lo(y) {}
+  __device__ __forceinline__ explicit operator float() const {
+    return isfinite(lo) ? hi + lo : hi;  // an infinite sum has no error term
+  }
+  friend __device__ __forceinline__ FloatPair op_add(FloatPair a, FloatPair b) {
+    const float s = a.hi + b.hi;  // Knuth's two-sum
+    const float bb = s - a.hi;
+    return FloatPair(s, (a.hi - (s - bb)) + (b.hi - bb) + (a.lo + b.lo));
+  }
+  friend __device__ __forceinline__ FloatPair shfl_xor(FloatPair v, int m) {
+    return FloatPair(__shfl_xor_sync(0xffffffffu, v.hi, m), __shfl_xor_sync(0xffffffffu, v.lo, m));
+  }
+};
+template <typename T> using SumOf = std::conditional_t<std::is_same_v<T, float>, FloatPair, T>;
+__device__ __forceinline__ int32_t load_sum(const int32_t *p) { return __ldcg(p); }
+__device__ __forceinline__ int64_t load_sum(const int64_t *p) {
+  return __ldcg(reinterpret_cast<const long long *>(p));
+}
+__device__ __forceinline__ FloatPair load_sum(const FloatPair *p) {
+  const float2 v = __ldcg(reinterpret_cast<const float2 *>(p));
+  return FloatPair(v.x, v.y);
+}
+
+template <typename T, int CH>
+__device__ __forceinline__ void load_chunks(Chunk<T> (&c)[CH], const T *in, int64_t base, int count,
+                                            bool vec) {
+  constexpr int E = Chunk<T>::E;
+#pragma unroll
+  for (int k = 0; k < CH; ++k) {
+    const int first = (k * static_cast<int>(blockDim.x) + static_cast<int>(threadIdx.x)) * E;
+    if (vec && first + E <= count) {
+      c[k].raw = __ldcg(reinterpret_cast<const uint4 *>(in + base + first));
+    } else {
+#pragma unroll
+      for (int e = 0; e < E; ++e)
+        c[k].e[e] = first + e < count ? in[base + first + e] : zero_of<T>();
+    }
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(TwoShape<T>::kThreads)
+    scan_sums_kernel(const T *in, int64_t n, SumOf<T> *sums, bool vec) {
+  asm volatile("griddepcontrol.launch_dependents;");
+  using P = TwoShape<T>;
+  constexpr int CH = P::kChunks;
+  constexpr int64_t kTile = P::S::kTile;
+  const int64_t base = static_cast<int64_t>(blockIdx.x) * kTile;
+  Chunk<T> c[CH];
+  load_chunks<T, CH>(c, in, base, static_cast<int>(min64(kTile, n - base)), vec);
+  SumOf<T> acc = SumOf<T>(0);
+#pragma unroll
+  for (int k = 0; k < CH; ++k) {
+    T s = op_add(c[k].e[0], c[k].e[1]);
+    if (Chunk<T>::E == 4) s = op_add(s, op_add(c[k].e[Chunk<T>::E - 2], c[k].e[Chunk<T>::E - 1]));
+    acc = op_add(acc, SumOf<T>(s));
+  }
+  acc = warp_sum(acc);
+  __shared__ SumOf<T> ws[P::kWarps];
+  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = acc;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    SumOf<T> v = threadIdx.x < P::kWarps ? ws[threadIdx.x] : SumOf<T>(0);
+    v = warp_sum(v);
+    if (threadIdx.x == 0) sums[blockIdx.x] = v;
+  }
+}
+
+template <typename T, bool kInclusive>
+__global__ void __launch_bounds__(TwoShape<T>::kThreads, TwoShape<T>::kBlocks)
+    scan_tiles_kernel(const T *in, T *out, int64_t n, const SumOf<T> *sums, bool vec_in,
+                      bool vec_out) {
+  using P = TwoShape<T>;
+  using S = typename P::S;
+  constexpr int CH = P::kChunks;
+  __shared__ typename S::Shared sh;
+  __shared__ SumOf<T> part[P::kWarps];
+  const int t = threadIdx.x, lane = t & 31;
+  const int64_t base = static_cast<int64_t>(blockIdx.x) * S::kTile;
+  const int count = static_cast<int>(min64(S::kTile, n - base));
+  Chunk<T> c[CH];
+  load_chunks<T, CH>(c, in, base, count, vec_in);
+  T wex[CH];
+  S::scan_chunks(c, wex, sh);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  SumOf<T> v = SumOf<T>(0);
+  for (unsigned j = t; j < blockIdx.x; j += P::kThreads) v = op_add(v, load_sum(sums + j));
+  v = warp_sum(v);
+  if (lane == 0) part[t >> 5] = v;
+  __syncthreads();
+  if (t < 32) {
+    S::phase2_warp0(sh, lane);
+    v = lane < P::kWarps ? part[lane] : SumOf<T>(0);
+    v = warp_sum(v);
+    if (lane == 0) sh.prefix = T(v);
+  }
+  __syncthreads();
+  S::template phase3<kInclusive>(c, wex, sh, sh.prefix);
+  S::template store<true>(out, base, count, c, vec_out);
+}
+
+template <typename T, bool kInclusive>
+int launch_two(const T *in, T *out, int64_t n, char *w, cudaStream_t st) {
+  constexpr int64_t kTile = TwoShape<T>::S::kTile;
+  const unsigned tiles = static_cast<unsigned>((n + kTile - 1) / kTile);
+  SumOf<T> *sums = reinterpret_cast<SumOf<T> *>(w);
+  scan_sums_kernel<T><<<tiles, TwoShape<T>::kThreads, 0, st>>>(in, n, sums, aligned16(in));
+  const int s = launch_status();
+  if (s != EDPP_OK) return s;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(tiles);
+  cfg.blockDim = dim3(TwoShape<T>::kThreads);
+  cfg.stream = st;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cuda_status(cudaLaunchKernelEx(&cfg, scan_tiles_kernel<T, kInclusive>, in, out, n,
+                                        static_cast<const SumOf<T> *>(sums), aligned16(in),
+                                        aligned16(out)));
+}
+
+// The longest input of the two-launch form.  Beyond it the second read finds less
+// and less of the input in L2, and the pipelined scan, which reads once, is ahead:
+// int32 48 MB 23.3 us against 25.1, 64 MB 32.8 against 31.9; int64 32 MB 22.8 against
+// 24.1, 48 MB 31.2 against 29.0.
+template <typename T> constexpr int64_t two_max() {
+  return (sizeof(T) == 4 ? 48ll << 20 : 32ll << 20) / static_cast<int64_t>(sizeof(T));
 }
 
 // ---- RTS / SSA building blocks ----------------------------------------------
@@ -768,11 +931,12 @@ int scan_impl(const T *in, T *out, int64_t n, int algo, void *ws, size_t ws_byte
   const bool vec_out = aligned16(out);
   char *w = static_cast<char *>(ws);
 
-  if (variant < 0 && algo != EDPP_SCAN_SSA && n <= small_max<T>())
+  if (variant < 0 && algo != EDPP_SCAN_SSA && n <= two_max<T>()) {
     variant = chosen_variant(
         algo == EDPP_SCAN_LOOKBACK ? EDPP_TUNE_SCAN_LOOKBACK : EDPP_TUNE_SCAN_RTS, sizeof(T), n);
-  if (variant < 0 && algo != EDPP_SCAN_SSA && n <= small_max<T>())
-    return launch_small<T, kInclusive>(in, out, n, st);
+    if (variant < 0 && n <= small_max<T>()) return launch_small<T, kInclusive>(in, out, n, st);
+    if (variant < 0 && aligned16(w)) return launch_two<T, kInclusive>(in, out, n, w, st);
+  }
   if (algo == EDPP_SCAN_LOOKBACK) {
     if (variant < 0) variant = tuned_variant(EDPP_TUNE_SCAN_LOOKBACK, sizeof(T), n, 0);
     switch (variant) {

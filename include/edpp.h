@@ -508,8 +508,9 @@ typedef enum {
 /* Number of variants of a primitive (0: not tunable). */
 int edpp_tune_variants(int primitive);
 /* Record `variant` (measured at `ms`, informational) for the class.  Look-back
- * and reduce-then-scan calls of up to 512 KB, which otherwise run in one
- * thread-block cluster whatever the table holds, take a variant set here. */
+ * and reduce-then-scan calls of up to 512 KB (one thread-block cluster) and 48
+ * MB (64-bit elements: 32 MB; two launches), which otherwise run in those forms
+ * whatever the table holds, take a variant set here. */
 int edpp_tune_set(int primitive, int elem_bytes, int log2_length, int variant, float ms);
 /* The variant a call of `length` elements takes now (EDPP_OK), or the
  * default with EDPP_EINVAL when the table has no entry for the primitive. */
