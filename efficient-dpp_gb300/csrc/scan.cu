@@ -196,10 +196,14 @@ __global__ void __launch_bounds__(kSmallThreads)
   __syncwarp();
   cluster_arrive();  // all sums have arrived, and warp_pre is visible to the block
   cluster_wait();
-  T prefix = zero_of<T>();
+  T before[kSmallBlocks];
 #pragma unroll
-  for (unsigned r = 0; r + 1 < kSmallBlocks; ++r)
-    if (r < b) prefix = op_add(prefix, sums[r]);
+  for (unsigned r = 0; r < kSmallBlocks; ++r) before[r] = r < b ? sums[r] : zero_of<T>();
+#pragma unroll
+  for (int d = 1; d < kSmallBlocks; d *= 2)  // pairwise: three roundings of a float sum, not seven
+#pragma unroll
+    for (int r = 0; r < kSmallBlocks; r += 2 * d) before[r] = op_add(before[r], before[r + d]);
+  const T prefix = before[0];
   S::template phase3<kInclusive>(c, wex, sh, prefix);
   S::store(out, base, count, c, vec_out);
 }
