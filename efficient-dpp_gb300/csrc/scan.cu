@@ -130,15 +130,16 @@ __global__ void __launch_bounds__(TH, MINB)
 }
 
 // ---- small inputs: one thread-block cluster ----------------------------------
-// Up to kSmallBlocks tiles of 32 or 64 KB, one per block of a cluster: a block
+// Up to kSmallBlocks tiles of 32 KB, one per block of a cluster: a block
 // scans its tile in registers, writes the tile's sum into the shared memory of
 // every block of the cluster, and after one cluster barrier adds up the sums
 // before its own.  No state in global memory, so no memset ahead of the launch
 // and no look-back: bound by launch and load latency.  Device time of one call
 // among others in a graph, int32: 1000 elements 6.3 -> 2.3 us, 65536 6.4 -> 3.0
-// (reduce-then-scan 8.3 -> 3.0), 131072 6.8 -> 3.8.
-constexpr int kSmallThreads = 512, kSmallBlocks = 8;
-template <typename T, int CH> using TSS = TileScan<T, kSmallThreads, CH>;
+// (reduce-then-scan 8.3 -> 3.0).  From there on (tiles of 64 KB: 3.9) the two
+// launches below take 3.7.
+constexpr int kSmallThreads = 512, kSmallChunks = 4, kSmallBlocks = 8;
+template <typename T> using TSS = TileScan<T, kSmallThreads, kSmallChunks>;
 
 // Shared-memory store into block `rank` of the cluster.
 __device__ __forceinline__ void st_cluster(void *p, unsigned rank, uint64_t bits, int bytes) {
@@ -158,10 +159,11 @@ __device__ __forceinline__ void cluster_wait() {
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-template <typename T, bool kInclusive, int CH>
+template <typename T, bool kInclusive>
 __global__ void __launch_bounds__(kSmallThreads)
     scan_small_kernel(const T *in, T *out, int64_t n, bool vec_in, bool vec_out) {
-  using S = TSS<T, CH>;
+  using S = TSS<T>;
+  constexpr int CH = kSmallChunks;
   constexpr int E = Chunk<T>::E;
   __shared__ typename S::Shared sh;
   __shared__ T sums[kSmallBlocks];
@@ -208,9 +210,9 @@ __global__ void __launch_bounds__(kSmallThreads)
   S::store(out, base, count, c, vec_out);
 }
 
-template <typename T, bool kInclusive, int CH>
-int launch_small_as(const T *in, T *out, int64_t n, cudaStream_t st) {
-  const unsigned blocks = static_cast<unsigned>((n + TSS<T, CH>::kTile - 1) / TSS<T, CH>::kTile);
+template <typename T, bool kInclusive>
+int launch_small(const T *in, T *out, int64_t n, cudaStream_t st) {
+  const unsigned blocks = static_cast<unsigned>((n + TSS<T>::kTile - 1) / TSS<T>::kTile);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(blocks);
   cfg.blockDim = dim3(kSmallThreads);
@@ -221,18 +223,12 @@ int launch_small_as(const T *in, T *out, int64_t n, cudaStream_t st) {
   attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  return cuda_status(cudaLaunchKernelEx(&cfg, scan_small_kernel<T, kInclusive, CH>, in, out, n,
+  return cuda_status(cudaLaunchKernelEx(&cfg, scan_small_kernel<T, kInclusive>, in, out, n,
                                         aligned16(in), aligned16(out)));
 }
 
-// The longest input of the cluster form.
-template <typename T> constexpr int64_t small_max() { return kSmallBlocks * TSS<T, 8>::kTile; }
-
-template <typename T, bool kInclusive>
-int launch_small(const T *in, T *out, int64_t n, cudaStream_t st) {
-  return n <= kSmallBlocks * TSS<T, 4>::kTile ? launch_small_as<T, kInclusive, 4>(in, out, n, st)
-                                              : launch_small_as<T, kInclusive, 8>(in, out, n, st);
-}
+// The longest input of the cluster form (256 KB).
+template <typename T> constexpr int64_t small_max() { return kSmallBlocks * TSS<T>::kTile; }
 
 // ---- middle sizes: two launches, one tile per block ----------------------------
 // scan_sums adds up every tile; scan_tiles scans them, each block adding up the

@@ -508,7 +508,7 @@ typedef enum {
 /* Number of variants of a primitive (0: not tunable). */
 int edpp_tune_variants(int primitive);
 /* Record `variant` (measured at `ms`, informational) for the class.  Look-back
- * and reduce-then-scan calls of up to 512 KB (one thread-block cluster) and 48
+ * and reduce-then-scan calls of up to 256 KB (one thread-block cluster) and 48
  * MB (64-bit elements: 32 MB; two launches), which otherwise run in those forms
  * whatever the table holds, take a variant set here. */
 int edpp_tune_set(int primitive, int elem_bytes, int log2_length, int variant, float ms);

@@ -1,4 +1,4 @@
-"""The two-launch scan of middle sizes (512 KB to 48 MB, 64-bit 32 MB) at the
+"""The two-launch scan of middle sizes (256 KB to 48 MB, 64-bit 32 MB) at the
 edges of its range, of its tiles (32 KB) and of the strides in which the tile
 sums are added up; unaligned and in place; infinities and NaN; captured in a
 CUDA graph; on two streams at once."""
@@ -6,7 +6,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-TILE_BYTES, SMALL_BYTES = 32768, 512 << 10
+TILE_BYTES, SMALL_BYTES = 32768, 256 << 10
 
 
 def _lengths(elem):
