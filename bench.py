@@ -414,9 +414,10 @@ def measure_batch(args, dev, world, steps, warmup, autotune=False):
     ops = {B.OP_NAMES[k]: int((segs["op"] == k).sum()) for k in (0, 1, 2)}
     kinds = tuning is None or tuning.schedule == B.SCHEDULE_KINDS
     # kernels per batch: KINDS launches one kernel per tile kind present
-    # (a split takes three: histogram, per-segment histogram scans, scatter)
-    launches = (int(bool(ops["scan"])) + int(bool(ops["gather"])) + 3 * int(bool(ops["split"]))
-                if kinds else 1)
+    # (a split takes three: histogram, per-segment histogram scans, scatter;
+    # the scans share the gathers' launch)
+    launches = (int(bool(ops["scan"])) + int(bool(ops["gather"] or ops["split"])) +
+                2 * int(bool(ops["split"])) if kinds else 1)
     del d0, d1, o0, o1, q0, q1, ws, pws, qws
     torch.cuda.empty_cache()
     return {
