@@ -369,8 +369,8 @@ typedef struct {
 
 /* How a batch runs on the GPU:
  *   KINDS  one launch per kind of tile over every segment of that kind (scan
- *          tiles; gather tiles; split histogram tiles, the per-segment
- *          histogram scans, split scatter tiles), each sized for its kind
+ *          tiles; split histogram tiles; gather tiles and the per-segment
+ *          histogram scans; split scatter tiles), each sized for its kind
  *   QUEUE  one persistent launch whose blocks take all tiles from one work
  *          queue (blocks_per_sm, split_defer_segments, largest_first apply) */
 typedef enum {
