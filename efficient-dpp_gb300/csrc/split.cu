@@ -27,7 +27,8 @@
 // Inputs whose tiles are all resident at once (up to 2.4 million elements) take
 // one cooperative launch instead (the fused form of the scatter kernel): the
 // tile is read once, its counts come from its ranking, and the blocks exchange
-// them through his.
+// them through his.  With few tiles times buckets they take two plain launches:
+// the counts, then that kernel, which adds them up itself.
 //
 // Ranks follow input order inside a warp segment, warp segments follow
 // input order inside a tile, tiles follow input order in the scan: the split
@@ -66,6 +67,43 @@ template <int LAYOUT> __device__ __forceinline__ int32_t key_at(const int32_t *k
 }
 
 // ---- stage 1: per-tile bucket counts ----------------------------------------
+// Adds the keys of the tile at `base` to its bucket counts mine[] (shared).
+template <int LAYOUT, int TILE, int THREADS>
+__device__ __forceinline__ void count_tile(const int32_t *__restrict__ keys, int64_t base, int64_t n,
+                                           int shift, unsigned mask, bool vec, uint32_t *mine) {
+  const int count = static_cast<int>(min64(TILE, n - base));
+  auto add = [&](bool valid, int32_t key) {
+    if (valid) atomicAdd(&mine[(static_cast<unsigned>(key) >> shift) & mask], 1u);
+  };
+  if (LAYOUT != EDPP_KVS_AOS && vec && count == TILE) {
+    // 16-byte vectors, warp-contiguous: 4 keys per thread per step.
+    const int4 *k4 = reinterpret_cast<const int4 *>(keys + base);
+#pragma unroll (THREADS == kHistThreads ? 2 : 4)
+    for (int v = threadIdx.x; v < TILE / 4; v += THREADS) {
+      const int4 q = __ldcs(k4 + v);
+      add(true, q.x);
+      add(true, q.y);
+      add(true, q.z);
+      add(true, q.w);
+    }
+  } else if (LAYOUT == EDPP_KVS_AOS && vec && count == TILE) {
+    // 16-byte vectors of two pairs.
+    const int4 *p4 = reinterpret_cast<const int4 *>(keys + 2 * base);
+#pragma unroll (THREADS == kHistThreads ? 2 : 4)
+    for (int v = threadIdx.x; v < TILE / 2; v += THREADS) {
+      const int4 q = __ldcs(p4 + v);
+      add(true, q.x);
+      add(true, q.z);
+    }
+  } else {
+    for (int i0 = 0; i0 < count; i0 += THREADS) {
+      const int i = i0 + threadIdx.x;
+      const bool valid = i < count;
+      add(valid, valid ? key_at<LAYOUT>(keys, base + i) : 0);
+    }
+  }
+}
+
 // One block counts TP consecutive tiles.  Row b of his is `stride` long, tiles
 // rounded up to TP (the padding columns count zero).  Bound by DRAM up to 64
 // buckets; above, one 4-byte store per bucket and tile cost as much as the
@@ -86,38 +124,7 @@ __global__ void __launch_bounds__(kHistThreads)
   for (int j = 0; j < TP; ++j) {
     const int64_t base = (t0 + j) * TILE;
     if (base >= n) break;
-    const int count = static_cast<int>(min64(TILE, n - base));
-    uint32_t *mine = cnt + j * buckets;
-    auto add = [&](bool valid, int32_t key) {
-      if (valid) atomicAdd(&mine[(static_cast<unsigned>(key) >> shift) & mask], 1u);
-    };
-    if (LAYOUT != EDPP_KVS_AOS && vec && count == TILE) {
-      // 16-byte vectors, warp-contiguous: 4 keys per thread per step.
-      const int4 *k4 = reinterpret_cast<const int4 *>(keys + base);
-#pragma unroll 2
-      for (int v = threadIdx.x; v < TILE / 4; v += kHistThreads) {
-        const int4 q = __ldcs(k4 + v);
-        add(true, q.x);
-        add(true, q.y);
-        add(true, q.z);
-        add(true, q.w);
-      }
-    } else if (LAYOUT == EDPP_KVS_AOS && vec && count == TILE) {
-      // 16-byte vectors of two pairs.
-      const int4 *p4 = reinterpret_cast<const int4 *>(keys + 2 * base);
-#pragma unroll 2
-      for (int v = threadIdx.x; v < TILE / 2; v += kHistThreads) {
-        const int4 q = __ldcs(p4 + v);
-        add(true, q.x);
-        add(true, q.z);
-      }
-    } else {
-      for (int i0 = 0; i0 < count; i0 += kHistThreads) {
-        const int i = i0 + threadIdx.x;
-        const bool valid = i < count;
-        add(valid, valid ? key_at<LAYOUT>(keys, base + i) : 0);
-      }
-    }
+    count_tile<LAYOUT, TILE, kHistThreads>(keys, base, n, shift, mask, vec, cnt + j * buckets);
   }
   __syncthreads();
   for (int b = threadIdx.x; b < buckets; b += kHistThreads) {
@@ -173,15 +180,37 @@ size_t scatter_smem_bytes(int buckets, bool bulk = false) {
 // *fused.arrived (bounded wait) each block adds up what precedes its runs: the
 // smaller buckets' totals and its bucket's counts in the tiles before.  The
 // tile waits in registers meanwhile.
+//
+// Where few words are exchanged, the counts come from split_counts_kernel instead
+// (arrived null): two plain launches, no memset and no waiting among blocks.  The
+// second is programmatic, so it loads and ranks its tile while the first runs, and
+// waits for that one's end before it adds up.
 struct FusedArgs {
-  unsigned *arrived;      // zeroed before the launch
+  unsigned *arrived;      // zeroed before the launch; null: his is the counts kernel's
   int32_t *his;           // [tiles][buckets]
   int32_t *bucket_start;  // may be null
 };
 
+// The counts of tile t as row t of his, for the two-launch form.
+constexpr int kCountThreads = 512;
+template <int LAYOUT, int TILE>
+__global__ void __launch_bounds__(kCountThreads)
+    split_counts_kernel(const int32_t *__restrict__ keys, int64_t n, int buckets, int shift,
+                        int32_t *__restrict__ his, bool vec) {
+  __shared__ uint32_t cnt[kOnePassMax];
+  asm volatile("griddepcontrol.launch_dependents;");
+  for (int b = threadIdx.x; b < buckets; b += kCountThreads) cnt[b] = 0;
+  __syncthreads();
+  count_tile<LAYOUT, TILE, kCountThreads>(keys, static_cast<int64_t>(blockIdx.x) * TILE, n, shift,
+                           static_cast<unsigned>(buckets - 1), vec, cnt);
+  __syncthreads();
+  for (int b = threadIdx.x; b < buckets; b += kCountThreads)
+    his[static_cast<int64_t>(blockIdx.x) * buckets + b] = static_cast<int32_t>(cnt[b]);
+}
+
 // Output start of every bucket's run of tile t, into start[] (shared): publish
-// the tile's counts (cnt[], shared) as row t of his, wait for all tiles', add up
-// the rows.  A thread reads 16-byte quads 2048 words apart, which hold the same
+// the tile's counts (cnt[], shared) as row t of his unless they are there, wait
+// for all tiles', add up the rows.  A thread reads 16-byte quads 2048 words apart, which hold the same
 // buckets each time (the bucket counts divide 2048); tot[] is shared scratch.
 // False: the wait ran out.
 template <int THREADS>
@@ -194,24 +223,29 @@ __device__ __forceinline__ bool fused_starts(const FusedArgs &f, int t, int tile
   __shared__ int32_t s_sum[kWarps];
   __shared__ int s_ok;
   for (int b = tid; b < buckets; b += THREADS) {
-    f.his[t * buckets + b] = cnt[b];
+    if (f.arrived) f.his[t * buckets + b] = cnt[b];
     start[b] = 0;
     tot[b] = 0;
   }
-  __threadfence();
-  __syncthreads();
-  if (tid == 0) {
-    atomicAdd(f.arrived, 1u);
-    const uint64_t t0 = globaltimer_ns();
-    bool ok;
-    while (!(ok = ld_acquire_u32(f.arrived) >= static_cast<uint32_t>(tiles)) &&
-           globaltimer_ns() - t0 <= timeout_ns) {
+  if (f.arrived) {
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) {
+      atomicAdd(f.arrived, 1u);
+      const uint64_t t0 = globaltimer_ns();
+      bool ok;
+      while (!(ok = ld_acquire_u32(f.arrived) >= static_cast<uint32_t>(tiles)) &&
+             globaltimer_ns() - t0 <= timeout_ns) {
+      }
+      if (!ok) raise_fault(fault, EDPP_FAULT_TIMEOUT);
+      s_ok = ok ? 1 : 0;
     }
-    if (!ok) raise_fault(fault, EDPP_FAULT_TIMEOUT);
-    s_ok = ok ? 1 : 0;
+    __syncthreads();
+    if (!s_ok) return false;
+  } else {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    __syncthreads();
   }
-  __syncthreads();
-  if (!s_ok) return false;
   const int words = tiles * buckets, mine = t * buckets;
   int32_t total[4] = {0, 0, 0, 0}, before[4] = {0, 0, 0, 0};
 #pragma unroll 8
@@ -782,6 +816,46 @@ int launch_fused(const SplitArgs &a, char *ws, cudaStream_t st) {
   return launch_status();
 }
 
+// The two-launch split with tiles of TILE elements.
+template <int LAYOUT, int TILE>
+int launch_counted(const SplitArgs &a, char *ws, cudaStream_t st) {
+  constexpr auto index = split_index_kernel<LAYOUT, TILE, true>;
+  constexpr auto scatter = split_scatter_kernel<kScatterThreads, LAYOUT, TILE, true>;
+  const bool by_index = a.buckets >= index_buckets<LAYOUT>();
+  int s = by_index
+              ? prepare_kernel<index>(kIndexThreads, index_smem_bytes<LAYOUT, TILE>(kOnePassMax),
+                                      nullptr)
+              : prepare_kernel<scatter>(kScatterThreads,
+                                        scatter_smem_bytes<kScatterThreads, LAYOUT, TILE>(
+                                            index_buckets<LAYOUT>(), true),
+                                        nullptr);
+  if (s != EDPP_OK) return s;
+  const int64_t tiles = (a.n + TILE - 1) / TILE;
+  int32_t *counts = reinterpret_cast<int32_t *>(ws);
+  split_counts_kernel<LAYOUT, TILE><<<static_cast<unsigned>(tiles), kCountThreads, 0, st>>>(
+      a.keys_in, a.n, a.buckets, a.shift, counts, aligned16(a.keys_in));
+  s = launch_status();
+  if (s != EDPP_OK) return s;
+  const FusedArgs fused{nullptr, counts, a.bucket_start};
+  const bool flag = by_index ? a.exact : bulk_runs<LAYOUT>(a);
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(tiles));
+  cfg.blockDim = dim3(by_index ? kIndexThreads : kScatterThreads);
+  cfg.dynamicSmemBytes = by_index
+                             ? index_smem_bytes<LAYOUT, TILE>(a.buckets)
+                             : scatter_smem_bytes<kScatterThreads, LAYOUT, TILE>(a.buckets, flag);
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  const int32_t *his = nullptr;
+  return cuda_status(cudaLaunchKernelEx(
+      &cfg, by_index ? index : scatter, a.keys_in, a.keys_out, a.vals_in, a.vals_out, a.n,
+      a.buckets, a.shift, tiles, his, a.tma, flag, kDefaultWaitNs, fault_word(), fused));
+}
+
 // The fused form takes an input when its tiles are all resident (two blocks per
 // SM) and the words every block adds up are few: device time, three launches
 // against fused, key/value pairs: 256 buckets 10^5 pairs 20.6 -> 12.7 us, 10^6
@@ -792,6 +866,15 @@ int launch_fused(const SplitArgs &a, char *ws, cudaStream_t st) {
 // 20.6.
 constexpr int64_t kFusedWords = 1 << 16;
 constexpr int kSmallTile = 2048, kMidTile = 4096;
+
+// Up to this many words the counts come from a launch of their own, in tiles that
+// leave one or two blocks per SM.  Calls issued one after another / device time in
+// a graph, one cooperative launch against two plain ones, key/value pairs: 2 buckets
+// 10^5 10.4 / 10.3 -> 8.2 / 5.6 us, 16 buckets 6*10^5 11.6 / 12.1 -> 10.5 / 7.8, 10^6
+// 14.7 / 14.4 -> 12.6 / 9.9, 2*10^6 18.8 / 18.5 -> 16.8 / 14.3.  Above, the second
+// launch costs a caller's loop what it saves the device: 64 buckets 10^6 (15680
+// words) 14.6 / 14.4 -> 14.8 / 12.7, 256 buckets (62720) 16.7 / 16.5 -> 18.9 / 16.3.
+constexpr int64_t kCountedWords = 1 << 13;
 
 // Workspace of the fused form (256 bytes for the counter, then his), an upper
 // bound over its tile sizes.
@@ -806,6 +889,14 @@ template <int LAYOUT> int split_fused(const SplitArgs &a, char *ws, cudaStream_t
     const int64_t tiles = (a.n + tile - 1) / tile;
     return tiles <= blocks && tiles * a.buckets <= kFusedWords;
   };
+  auto counted = [&](int64_t tile, int64_t blocks) {
+    const int64_t tiles = (a.n + tile - 1) / tile;
+    return tiles <= blocks && tiles * a.buckets <= kCountedWords;
+  };
+  if (counted(kSmallTile, 2 * sms)) return launch_counted<LAYOUT, kSmallTile>(a, ws, st);
+  if (counted(kMidTile, 2 * sms)) return launch_counted<LAYOUT, kMidTile>(a, ws, st);
+  if (counted(kTile, 2 * sms) && !fits(kMidTile, 2 * sms))
+    return launch_counted<LAYOUT, kTile>(a, ws, st);
   if (fits(kSmallTile, sms)) return launch_fused<LAYOUT, kSmallTile>(a, ws, st);
   if (fits(kMidTile, sms)) return launch_fused<LAYOUT, kMidTile>(a, ws, st);
   if (fits(kTile, 2 * sms)) return launch_fused<LAYOUT, kTile>(a, ws, st);

@@ -104,3 +104,18 @@ def test_workspace_off_16_bytes(cuda, edpp, n):
     k, v, st = edpp.split(keys, 256, values=vals, bucket_start=True, ws=ws)
     assert cuda.equal(k, wk) and cuda.equal(v, wv) and cuda.equal(st, s)
     assert edpp.sync_status() == edpp.EDPP_OK
+
+
+@pytest.mark.parametrize("layout", ["ko", "soa", "aos"])
+@pytest.mark.parametrize("buckets", [1, 8, 16, 64, 256, 1024])
+def test_counts_launch_edges(cuda, edpp, buckets, layout):
+    # few words (2^13): the counts by a launch of their own, two tiles per SM at most
+    sms = cuda.cuda.get_device_properties(0).multi_processor_count
+    lengths = set()
+    for tile in (2048, 4096, 8192):
+        last = tile * min(2 * sms, (1 << 13) // buckets)
+        lengths |= {last - 1, last, last + 1}
+    for n in sorted(lengths):
+        _check(edpp, cuda, n, buckets, layout)
+        _check(edpp, cuda, n, buckets, layout, skew=True)
+    assert edpp.sync_status() == edpp.EDPP_OK
