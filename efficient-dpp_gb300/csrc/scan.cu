@@ -1107,6 +1107,18 @@ int edpp_selftest_lookback_timeout(const int32_t *in, int32_t *out, int64_t leng
                                          /*tile_base=*/1, timeout_ns, /*variant=*/0);
 }
 
+int edpp_selftest_scan_pipe_timeout(const int32_t *in, int32_t *out, int64_t length,
+                                    uint64_t timeout_ns, void *ws, size_t ws_bytes, void *stream) {
+  using namespace edpp;
+  if (length <= 0 || timeout_ns == 0 || !in || !out || !aligned16(in) || !aligned16(out))
+    return EDPP_EINVAL;
+  if (!ws || ws_bytes < workspace_bytes<int32_t>(length, EDPP_SCAN_LOOKBACK)) return EDPP_ENOMEM;
+  unsigned *fault = fault_word();
+  if (!fault) return EDPP_ECUDA;
+  return scan_pipe<int32_t, false>(in, out, length, static_cast<char *>(ws), as_stream(stream),
+                                   timeout_ns, fault, /*withheld=*/0);
+}
+
 }  // extern "C"
 
 // ---- allocation-free exclusive scan -------------------------------------------

@@ -112,10 +112,11 @@ struct TileAt {
   int32_t count, head;
 };
 
-// One array cut into tiles.
+// One array cut into tiles.  The sum of tile `withheld` is never published (the
+// bounded-wait self-test; -1 otherwise).
 template <typename T> struct ArrayTiles {
   static constexpr bool kSegmented = false;
-  int64_t n, num_tiles;
+  int64_t n, num_tiles, withheld;
   __device__ __forceinline__ TileAt at(int64_t tile) const {
     constexpr int kTile = kTileBytes / sizeof(T);
     return {tile * kTile, static_cast<int32_t>(min64(kTile, n - tile * kTile)), 0};
@@ -322,7 +323,9 @@ __global__ void __launch_bounds__(kThreads, 1)
       __syncwarp();
       if (lane == 0) mbar_arrive(&sh.empty[s]);
       const T v = warp_sum(acc[0]);
-      if (lane == 0) st.publish(i * G + b, flag, v);
+      bool known = lane == 0;
+      if constexpr (!kSegmented) known = known && i * G + b != tiles.withheld;
+      if (known) st.publish(i * G + b, flag, v);
     }
   } else if (warp == kScanWarps + kReduceWarps) {
     // ---- load ----
@@ -376,11 +379,12 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (bytes) tma_load_1d(buf(s), in + base, bytes, &sh.full[s]);
       }
     }
-    // after an abort the copies in flight land before the block's memory goes
-    if (i < steps)
-      for (int64_t j = max64(0, i - stages); j < i; ++j)
-        mbar_wait_bounded(&sh.full[j % stages], static_cast<uint32_t>(j / stages) & 1u, timeout_ns,
-                          fault);
+    // The copies in flight land before the block's memory goes, also when the
+    // last one is out and an abort sends every other role home: nobody else
+    // waits for them then.  Not within the call's limit, which may have run out.
+    for (int64_t j = max64(0, i - stages); j < i; ++j)
+      mbar_wait_bounded(&sh.full[j % stages], static_cast<uint32_t>(j / stages) & 1u,
+                        kDefaultWaitNs, fault);
   } else {
     // ---- prefix: warp q takes steps q, q + kPrefixWarps, ..., so the reads of
     // several waves overlap; the sum of the earlier waves passes from warp to
@@ -512,10 +516,10 @@ template <typename T> size_t scan_pipe_state_bytes(int64_t n) {
 
 template <typename T, bool kInclusive>
 int scan_pipe(const T *in, T *out, int64_t n, char *header, cudaStream_t st, uint64_t timeout_ns,
-              unsigned *fault) {
+              unsigned *fault, int64_t withheld) {
   if (!pipe_fits<T, kInclusive, ArrayTiles<T>>()) return EDPP_ENOMEM;
   constexpr int64_t kTile = kTileBytes / sizeof(T);
-  const ArrayTiles<T> tiles{n, (n + kTile - 1) / kTile};
+  const ArrayTiles<T> tiles{n, (n + kTile - 1) / kTile, withheld};
   if (cudaMemsetAsync(header, 0, kHeader + LookbackState<T>::bytes(tiles.num_tiles), st) !=
       cudaSuccess)
     return EDPP_ECUDA;
@@ -535,9 +539,9 @@ int scan_pipe_tasks(const int32_t *in, int32_t *out, const DevSeg *segs, const D
 #define EDPP_PIPE(T)                                                                             \
   template size_t scan_pipe_state_bytes<T>(int64_t);                                             \
   template int scan_pipe<T, false>(const T *, T *, int64_t, char *, cudaStream_t, uint64_t,      \
-                                   unsigned *);                                                  \
+                                   unsigned *, int64_t);                                         \
   template int scan_pipe<T, true>(const T *, T *, int64_t, char *, cudaStream_t, uint64_t,       \
-                                  unsigned *);
+                                  unsigned *, int64_t);
 EDPP_PIPE(int32_t)
 EDPP_PIPE(int64_t)
 EDPP_PIPE(float)

@@ -15,10 +15,11 @@ template <typename T> size_t scan_pipe_state_bytes(int64_t n);
 // Scan of n > 0 elements; in and out 16-byte aligned, in == out allowed.
 // `header`: 256 bytes of the workspace, zeroed here with the state after it;
 // the abort flag is at header + 8.  EDPP_ENOMEM (nothing launched) when the
-// grid cannot be resident together on this device.
+// grid cannot be resident together on this device.  `withheld`: a tile whose sum
+// is not published, so that the waits for it run out (self-test).
 template <typename T, bool kInclusive>
 int scan_pipe(const T *in, T *out, int64_t n, char *header, cudaStream_t st, uint64_t timeout_ns,
-              unsigned *fault);
+              unsigned *fault, int64_t withheld = -1);
 
 struct DevSeg;
 struct DevTask;

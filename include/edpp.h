@@ -562,6 +562,13 @@ int edpp_selftest_lookback_timeout(const int32_t *in, int32_t *out,
                                    int64_t length, uint64_t timeout_ns,
                                    void *ws, size_t ws_bytes, void *stream);
 
+/* The same for the pipelined one-launch scan (in and out 16-byte aligned): the
+ * sum of the first tile is never published, so every block gives up and no
+ * element is written.  ws of edpp_scan_workspace_size for the look-back scan. */
+int edpp_selftest_scan_pipe_timeout(const int32_t *in, int32_t *out,
+                                    int64_t length, uint64_t timeout_ns,
+                                    void *ws, size_t ws_bytes, void *stream);
+
 #ifdef __cplusplus
 }
 #endif
