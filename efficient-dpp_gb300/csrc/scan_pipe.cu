@@ -124,8 +124,9 @@ template <typename T> struct ArrayTiles {
 };
 
 // The scan tiles of a batch: tile i is a task's tile of its segment, and every
-// segment's first tile is a head.  A task outside the plan's tables is recorded
-// and counts no elements.
+// segment's first tile is a head.  A task outside the plan's tables, or of a
+// segment off 16-byte alignment (the tables of another plan: a bulk copy would
+// fault there), is recorded and counts no elements.
 struct TaskTiles {
   static constexpr bool kSegmented = true;
   const DevSeg *segs;
@@ -139,7 +140,7 @@ struct TaskTiles {
     bool ok = t.seg >= 0 && t.seg < num_segs;
     DevSeg seg{};
     if (ok) seg = segs[t.seg];
-    ok = ok && t.tile >= 0 && t.tile < seg.tiles;
+    ok = ok && t.tile >= 0 && t.tile < seg.tiles && (seg.off & 3) == 0;
     if (!ok) raise_fault(fault, EDPP_FAULT_PLAN);
     if (!ok) return {0, 0, 1};
     const int64_t off = static_cast<int64_t>(t.tile) * kTile;
