@@ -210,6 +210,7 @@ __global__ void __launch_bounds__(kSmallThreads)
   S::store(out, base, count, c, vec_out);
 }
 
+// EDPP_ENOMEM (nothing launched): the cluster launch was refused.
 template <typename T, bool kInclusive>
 int launch_small(const T *in, T *out, int64_t n, cudaStream_t st) {
   const unsigned blocks = static_cast<unsigned>((n + TSS<T>::kTile - 1) / TSS<T>::kTile);
@@ -223,8 +224,12 @@ int launch_small(const T *in, T *out, int64_t n, cudaStream_t st) {
   attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  return cuda_status(cudaLaunchKernelEx(&cfg, scan_small_kernel<T, kInclusive>, in, out, n,
-                                        aligned16(in), aligned16(out)));
+  if (cudaLaunchKernelEx(&cfg, scan_small_kernel<T, kInclusive>, in, out, n, aligned16(in),
+                         aligned16(out)) != cudaSuccess) {
+    cudaGetLastError();  // no room for the cluster: the caller takes another form
+    return EDPP_ENOMEM;
+  }
+  return launch_status();
 }
 
 // The longest input of the cluster form (256 KB).
@@ -934,7 +939,10 @@ int scan_impl(const T *in, T *out, int64_t n, int algo, void *ws, size_t ws_byte
   if (variant < 0 && algo != EDPP_SCAN_SSA && n <= two_max<T>()) {
     variant = chosen_variant(
         algo == EDPP_SCAN_LOOKBACK ? EDPP_TUNE_SCAN_LOOKBACK : EDPP_TUNE_SCAN_RTS, sizeof(T), n);
-    if (variant < 0 && n <= small_max<T>()) return launch_small<T, kInclusive>(in, out, n, st);
+    if (variant < 0 && n <= small_max<T>()) {
+      const int s = launch_small<T, kInclusive>(in, out, n, st);
+      if (s != EDPP_ENOMEM) return s;
+    }
     if (variant < 0 && aligned16(w)) return launch_two<T, kInclusive>(in, out, n, w, st);
   }
   if (algo == EDPP_SCAN_LOOKBACK) {
