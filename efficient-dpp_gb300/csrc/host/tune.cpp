@@ -3,7 +3,9 @@
 //
 // Entries map (primitive, element size, log2 of the length) to a variant.
 // The primitives look their size up at call time (tuned_variant); a length
-// between recorded classes takes the nearest one.  The committed table,
+// between recorded classes takes the nearest one.  Lookups read what every
+// class resolves to, worked out when the table changes, so a call of a few
+// microseconds takes no lock.  The committed table,
 // efficient-dpp_gb300/tuning/plain_gb300.tsv, is read on first use from
 // beside the library's lib/ directory (found with dladdr).  The reference
 // picks its tunables by hand per device (opencl/test/test_scan_global.cpp:
@@ -31,16 +33,18 @@ namespace {
 struct Entry {
   int prim, elem, cls, variant;
   float ms;
-  bool set;  // by edpp_tune_set, not by a file or the autotuner
 };
 
 const char *const kNames[] = {"scan_lookback", "scan_rts", "gather"};
 constexpr int kPrims = 3;
+constexpr int kClasses = 63;
 
 std::mutex g_mu;
 std::vector<Entry> g_table;
-bool g_loaded = false;
-std::atomic<bool> g_any_set{false};  // an entry of g_table has `set`
+std::atomic<bool> g_loaded{false};
+// 1 + the variant of the nearest recorded class, 0 without one:
+// [primitive][4-, 8-byte elements][class].
+std::atomic<signed char> g_pick[kPrims][2][kClasses];
 
 int prim_of(const char *name) {
   for (int p = 0; p < kPrims; ++p)
@@ -58,9 +62,7 @@ int variants_of(int prim) {
 }
 
 int class_of(int64_t n) {
-  int c = 0;
-  while (c < 62 && (int64_t{1} << (c + 1)) <= n) ++c;
-  return c;
+  return n > 1 ? 63 - __builtin_clzll(static_cast<unsigned long long>(n)) : 0;
 }
 
 // efficient-dpp_gb300/tuning/plain_gb300.tsv, from this library's path
@@ -78,54 +80,17 @@ std::string default_path() {
   return pkg + "/tuning/plain_gb300.tsv";
 }
 
-void set_locked(int prim, int elem, int cls, int variant, float ms, bool set) {
-  if (set) g_any_set = true;
+void set_locked(int prim, int elem, int cls, int variant, float ms) {
   for (Entry &e : g_table)
     if (e.prim == prim && e.elem == elem && e.cls == cls) {
       e.variant = variant;
       e.ms = ms;
-      e.set = set;
       return;
     }
-  g_table.push_back({prim, elem, cls, variant, ms, set});
+  g_table.push_back({prim, elem, cls, variant, ms});
 }
 
-int load_locked(const std::string &path) {
-  g_table.clear();
-  g_any_set = false;
-  g_loaded = true;
-  if (path.empty()) return EDPP_OK;
-  FILE *f = std::fopen(path.c_str(), "r");
-  if (!f) return EDPP_OK;  // no table: every primitive takes its default
-  char line[256];
-  int status = EDPP_OK;
-  while (std::fgets(line, sizeof line, f)) {
-    char *hash = std::strchr(line, '#');
-    if (hash) *hash = '\0';
-    char name[64];
-    int elem = 0, cls = 0, variant = 0;
-    float ms = 0.0f;
-    const int got = std::sscanf(line, "%63s %d %d %d %f", name, &elem, &cls, &variant, &ms);
-    if (got <= 0) continue;  // blank or comment
-    const int prim = got >= 4 ? prim_of(name) : -1;
-    if (prim < 0 || (elem != 4 && elem != 8) || cls < 0 || cls > 62 || variant < 0 ||
-        variant >= variants_of(prim)) {
-      status = EDPP_EINVAL;  // a malformed line is skipped and reported
-      continue;
-    }
-    set_locked(prim, elem, cls, variant, got >= 5 ? ms : 0.0f, false);
-  }
-  std::fclose(f);
-  return status;
-}
-
-void ensure_loaded_locked() {
-  if (!g_loaded) load_locked(default_path());
-}
-
-const Entry *nearest_locked(int prim, int elem_bytes, int64_t length) {
-  ensure_loaded_locked();
-  const int cls = class_of(length);
+const Entry *nearest_locked(int prim, int elem_bytes, int cls) {
   const Entry *best = nullptr;
   for (const Entry &e : g_table) {
     if (e.prim != prim || e.elem != elem_bytes) continue;
@@ -136,19 +101,59 @@ const Entry *nearest_locked(int prim, int elem_bytes, int64_t length) {
   return best;
 }
 
+// After every change of g_table.
+void publish_locked() {
+  for (int prim = 0; prim < kPrims; ++prim)
+    for (int big = 0; big < 2; ++big)
+      for (int cls = 0; cls < kClasses; ++cls) {
+        const Entry *e = nearest_locked(prim, big ? 8 : 4, cls);
+        g_pick[prim][big][cls].store(static_cast<signed char>(e ? e->variant + 1 : 0),
+                                     std::memory_order_relaxed);
+      }
+  g_loaded.store(true, std::memory_order_release);
+}
+
+int load_locked(const std::string &path) {
+  g_table.clear();
+  int status = EDPP_OK;
+  // without a table every primitive takes its default
+  FILE *f = path.empty() ? nullptr : std::fopen(path.c_str(), "r");
+  char line[256];
+  while (f && std::fgets(line, sizeof line, f)) {
+    char *hash = std::strchr(line, '#');
+    if (hash) *hash = '\0';
+    char name[64];
+    int elem = 0, cls = 0, variant = 0;
+    float ms = 0.0f;
+    const int got = std::sscanf(line, "%63s %d %d %d %f", name, &elem, &cls, &variant, &ms);
+    if (got <= 0) continue;  // blank or comment
+    const int prim = got >= 4 ? prim_of(name) : -1;
+    if (prim < 0 || (elem != 4 && elem != 8) || cls < 0 || cls >= kClasses || variant < 0 ||
+        variant >= variants_of(prim)) {
+      status = EDPP_EINVAL;  // a malformed line is skipped and reported
+      continue;
+    }
+    set_locked(prim, elem, cls, variant, got >= 5 ? ms : 0.0f);
+  }
+  if (f) std::fclose(f);
+  publish_locked();
+  return status;
+}
+
+void ensure_loaded_locked() {
+  if (!g_loaded.load(std::memory_order_relaxed)) load_locked(default_path());
+}
+
 }  // namespace
 
 int tuned_variant(int prim, int elem_bytes, int64_t length, int fallback) {
-  std::lock_guard<std::mutex> lk(g_mu);
-  const Entry *e = nearest_locked(prim, elem_bytes, length);
-  return e ? e->variant : fallback;
-}
-
-int chosen_variant(int prim, int elem_bytes, int64_t length) {
-  if (!g_any_set.load(std::memory_order_acquire)) return -1;
-  std::lock_guard<std::mutex> lk(g_mu);
-  const Entry *e = nearest_locked(prim, elem_bytes, length);
-  return e && e->set ? e->variant : -1;
+  if (elem_bytes != 4 && elem_bytes != 8) return fallback;
+  if (!g_loaded.load(std::memory_order_acquire)) {
+    std::lock_guard<std::mutex> lk(g_mu);
+    ensure_loaded_locked();
+  }
+  const int pick = g_pick[prim][elem_bytes == 8][class_of(length)].load(std::memory_order_relaxed);
+  return pick ? pick - 1 : fallback;
 }
 
 }  // namespace edpp
@@ -159,12 +164,13 @@ int edpp_tune_variants(int primitive) { return edpp::variants_of(primitive); }
 
 int edpp_tune_set(int primitive, int elem_bytes, int log2_length, int variant, float ms) {
   if (primitive < 0 || primitive >= edpp::kPrims || (elem_bytes != 4 && elem_bytes != 8) ||
-      log2_length < 0 || log2_length > 62 || variant < 0 ||
+      log2_length < 0 || log2_length >= edpp::kClasses || variant < 0 ||
       variant >= edpp::variants_of(primitive))
     return EDPP_EINVAL;
   std::lock_guard<std::mutex> lk(edpp::g_mu);
   edpp::ensure_loaded_locked();
-  edpp::set_locked(primitive, elem_bytes, log2_length, variant, ms, true);
+  edpp::set_locked(primitive, elem_bytes, log2_length, variant, ms);
+  edpp::publish_locked();
   return EDPP_OK;
 }
 
@@ -204,8 +210,7 @@ int edpp_tune_save(const char *path) {
 void edpp_tune_clear(void) {
   std::lock_guard<std::mutex> lk(edpp::g_mu);
   edpp::g_table.clear();
-  edpp::g_any_set = false;
-  edpp::g_loaded = true;
+  edpp::publish_locked();
 }
 
 int edpp_autotune_plain(int primitive, const void *in, void *out, const int32_t *loc,
@@ -279,10 +284,7 @@ int edpp_autotune_plain(int primitive, const void *in, void *out, const int32_t 
   }
   *best_variant = best;
   if (best_ms) *best_ms = best_t;
-  std::lock_guard<std::mutex> lk(edpp::g_mu);
-  edpp::ensure_loaded_locked();
-  edpp::set_locked(primitive, elem_bytes, edpp::class_of(length), best, best_t, false);
-  return EDPP_OK;
+  return edpp_tune_set(primitive, elem_bytes, edpp::class_of(length), best, best_t);
 }
 
 }  // extern "C"

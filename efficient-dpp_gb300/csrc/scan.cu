@@ -50,18 +50,18 @@ constexpr size_t kHeader = 256;
 constexpr int64_t kMaxChunkBlocks = 8192;
 
 template <typename T> using TS = TileScan<T, kThreads, kChunks>;
-// Look-back tile shapes (threads per block, 16-byte chunks per thread, blocks
-// per SM for 4- / 8-byte elements), chosen per size class by the tuning
-// table (edpp_tune_*):
-//   variant 0  128 x 8   16 KB tiles, 12 / 8 blocks per SM (the default:
-//              fewer warps idle at the barrier while warp 0 looks back)
-//   variant 1  256 x 8   32 KB tiles,  6 / 4 blocks per SM (half the tiles,
-//              so half the look-backs)
+// Variants of the look-back scan, chosen per size class by the tuning table
+// (edpp_tune_*); tile shapes as threads per block x 16-byte chunks per thread:
+//   variant 0  the default: the form of the length (default_form below);
+//              variant 1 for arrays that form does not take
+//   variant 1  256 x 8   32 KB tiles,  6 / 4 blocks per SM for 4- / 8-byte
+//              elements (half the tiles of 128 x 8, so half the look-backs)
 //   variant 2  512 x 4   32 KB tiles,  6 / 4 blocks per SM
 //   variant 3  the pipelined one-launch scan (scan_pipe.cu) for 16-byte
 //              aligned arrays; variant 1 otherwise
-// Variant 0's tiles are the smallest; tile state and workspace are sized
-// for them, so every shape fits the same workspace.
+// The allocation-free scan and the bounded-wait self-test take 128 x 8 (16 KB,
+// 12 blocks per SM): the smallest tiles, for which tile state and workspace are
+// sized, so every shape fits the same workspace.
 constexpr int kLbThreads = 128;
 constexpr int kLbChunks = 8;
 constexpr int kLbVariants = 4;
@@ -650,8 +650,8 @@ __global__ void __launch_bounds__(kThreads)
 // bounded; a block that gives up raises EDPP_FAULT_TIMEOUT and sets the
 // call's abort flag so the others stop too.
 // kSliceTiles is the slice length in tiles, chosen per size class by the
-// tuning table: variant 0 (the default) two tiles, for arrays off 16-byte
-// alignment only (others take the pipelined scan_pipe.cu), variant 1 one tile,
+// tuning table: variant 0 (the default) two tiles, for arrays only that the form
+// of the length (default_form below) does not take, variant 1 one tile,
 // variant 2 four tiles (reduced in two rounds of eight 16-byte loads per
 // thread), variant 3 two tiles with L2 eviction hints (kHint: the reduce's
 // loads evict-last, the second read's bulk copies evict-first), variant 4
@@ -918,10 +918,28 @@ int launch_rts_chunked(const T *in, T *out, int64_t n, char *w, cudaStream_t st,
   return launch_status();
 }
 
-// variant < 0: the tuning table's choice for this size (else the default).
+// Variant 0 of both schemes: one cluster up to 256 KB, two launches up to two_max,
+// the pipelined scan beyond (or with a workspace off 16 bytes, for which the two
+// launches' sums are not laid out, from where its cooperative launch pays: 2^19
+// int32 look-back 11, pipelined 12 us, 2^20 13.7 and 11.9).  EDPP_ENOMEM (nothing
+// launched) for what none of them takes: arrays off 16-byte alignment, refused
+// launches.
+constexpr int64_t kPipeMin = 1 << 19;
+template <typename T, bool kInclusive>
+int default_form(const T *in, T *out, int64_t n, char *w, cudaStream_t st, unsigned *fault) {
+  if (n <= small_max<T>()) {
+    const int s = launch_small<T, kInclusive>(in, out, n, st);
+    if (s != EDPP_ENOMEM) return s;
+  }
+  if (n <= two_max<T>() && aligned16(w)) return launch_two<T, kInclusive>(in, out, n, w, st);
+  if (n <= kPipeMin || !aligned16(in) || !aligned16(out)) return EDPP_ENOMEM;
+  return scan_pipe<T, kInclusive>(in, out, n, w, st, kDefaultWaitNs, fault);
+}
+
+// variant < 0: the tuning table's choice for this size (else variant 0).
 template <typename T, bool kInclusive>
 int scan_impl(const T *in, T *out, int64_t n, int algo, void *ws, size_t ws_bytes, void *stream,
-              int64_t tile_base = 0, uint64_t timeout_ns = kDefaultWaitNs, int variant = -1) {
+              int variant = -1) {
   if (n < 0) return EDPP_EINVAL;
   if (algo != EDPP_SCAN_LOOKBACK && algo != EDPP_SCAN_RTS && algo != EDPP_SCAN_SSA)
     return EDPP_EINVAL;
@@ -934,49 +952,34 @@ int scan_impl(const T *in, T *out, int64_t n, int algo, void *ws, size_t ws_byte
   if (!fault) return EDPP_ECUDA;
   const bool tma = aligned16(in);
   const bool vec_out = aligned16(out);
+  const uint64_t timeout_ns = kDefaultWaitNs;
   char *w = static_cast<char *>(ws);
 
-  if (variant < 0 && algo != EDPP_SCAN_SSA && n <= two_max<T>()) {
-    variant = chosen_variant(
-        algo == EDPP_SCAN_LOOKBACK ? EDPP_TUNE_SCAN_LOOKBACK : EDPP_TUNE_SCAN_RTS, sizeof(T), n);
-    if (variant < 0 && n <= small_max<T>()) {
-      const int s = launch_small<T, kInclusive>(in, out, n, st);
+  if (algo != EDPP_SCAN_SSA) {
+    if (variant < 0)
+      variant = tuned_variant(
+          algo == EDPP_SCAN_LOOKBACK ? EDPP_TUNE_SCAN_LOOKBACK : EDPP_TUNE_SCAN_RTS, sizeof(T), n, 0);
+    if (variant == 0) {
+      const int s = default_form<T, kInclusive>(in, out, n, w, st, fault);
       if (s != EDPP_ENOMEM) return s;
     }
-    if (variant < 0 && aligned16(w)) return launch_two<T, kInclusive>(in, out, n, w, st);
   }
   if (algo == EDPP_SCAN_LOOKBACK) {
-    if (variant < 0) variant = tuned_variant(EDPP_TUNE_SCAN_LOOKBACK, sizeof(T), n, 0);
-    switch (variant) {
-      case 1:
-        return launch_lookback<T, kInclusive, 256, 8, 6, 4>(in, out, n, w, st, tile_base, tma,
-                                                            vec_out, timeout_ns, fault);
-      case 2:
-        return launch_lookback<T, kInclusive, 512, 4, 6, 4>(in, out, n, w, st, tile_base, tma,
-                                                            vec_out, timeout_ns, fault);
-      case 3: {
-        const int s = tma && vec_out ? scan_pipe<T, kInclusive>(in, out, n, w, st, timeout_ns, fault)
-                                     : EDPP_ENOMEM;
-        if (s != EDPP_ENOMEM) return s;
-        return launch_lookback<T, kInclusive, 256, 8, 6, 4>(in, out, n, w, st, tile_base, tma,
-                                                            vec_out, timeout_ns, fault);
-      }
-      default:
-        return launch_lookback<T, kInclusive, kLbThreads, kLbChunks, 12, 8>(
-            in, out, n, w, st, tile_base, tma, vec_out, timeout_ns, fault);
+    if (variant == 3 && tma && vec_out) {
+      const int s = scan_pipe<T, kInclusive>(in, out, n, w, st, timeout_ns, fault);
+      if (s != EDPP_ENOMEM) return s;
     }
+    if (variant == 2)
+      return launch_lookback<T, kInclusive, 512, 4, 6, 4>(in, out, n, w, st, 0, tma, vec_out,
+                                                          timeout_ns, fault);
+    return launch_lookback<T, kInclusive, 256, 8, 6, 4>(in, out, n, w, st, 0, tma, vec_out,
+                                                        timeout_ns, fault);
   }
 
   int64_t blocks, tpb;
   chunk_grid<T>(n, blocks, tpb);
   T *partials = reinterpret_cast<T *>(w + kHeader);
   const int64_t per = tpb * TS<T>::kTile;
-  if (algo == EDPP_SCAN_RTS && variant < 0)
-    variant = tuned_variant(EDPP_TUNE_SCAN_RTS, sizeof(T), n, 0);
-  if (algo == EDPP_SCAN_RTS && variant == 0 && tma && vec_out) {
-    const int s = scan_pipe<T, kInclusive>(in, out, n, w, st, timeout_ns, fault);
-    if (s != EDPP_ENOMEM) return s;
-  }
   if (algo == EDPP_SCAN_RTS && variant != 4 &&
       static_cast<double>(n) * sizeof(T) <= 0.6 * static_cast<double>(device_l2_bytes())) {
     // the input stays in L2 between the reduce and the scan: one launch
@@ -1055,12 +1058,10 @@ int scan_with_variant(const void *in, void *out, int64_t length, int elem_bytes,
   if (variant < 0 || variant >= scan_variants(algo)) return EDPP_EINVAL;
   if (elem_bytes == 4)
     return scan_impl<int32_t, false>(static_cast<const int32_t *>(in), static_cast<int32_t *>(out),
-                                     length, algo, ws, ws_bytes, stream, 0, kDefaultWaitNs,
-                                     variant);
+                                     length, algo, ws, ws_bytes, stream, variant);
   if (elem_bytes == 8)
     return scan_impl<int64_t, false>(static_cast<const int64_t *>(in), static_cast<int64_t *>(out),
-                                     length, algo, ws, ws_bytes, stream, 0, kDefaultWaitNs,
-                                     variant);
+                                     length, algo, ws, ws_bytes, stream, variant);
   return EDPP_EINVAL;
 }
 
@@ -1108,11 +1109,16 @@ int edpp_scan_inclusive_f32(const float *in, float *out, int64_t length, int alg
 
 int edpp_selftest_lookback_timeout(const int32_t *in, int32_t *out, int64_t length,
                                    uint64_t timeout_ns, void *ws, size_t ws_bytes, void *stream) {
-  if (length <= 0 || timeout_ns == 0) return EDPP_EINVAL;
+  using namespace edpp;
+  if (length <= 0 || timeout_ns == 0 || !in || !out) return EDPP_EINVAL;
+  if (!ws || ws_bytes < workspace_bytes<int32_t>(length, EDPP_SCAN_LOOKBACK)) return EDPP_ENOMEM;
+  unsigned *fault = fault_word();
+  if (!fault) return EDPP_ECUDA;
   // Tickets start at tile 1: tile 0 is never scanned, so tile 1 (and every
   // later tile) waits for a prefix nobody publishes until the limit runs out.
-  return edpp::scan_impl<int32_t, false>(in, out, length, EDPP_SCAN_LOOKBACK, ws, ws_bytes, stream,
-                                         /*tile_base=*/1, timeout_ns, /*variant=*/0);
+  return launch_lookback<int32_t, false, kLbThreads, kLbChunks, 12, 8>(
+      in, out, length, static_cast<char *>(ws), as_stream(stream), /*tile_base=*/1, aligned16(in),
+      aligned16(out), timeout_ns, fault);
 }
 
 int edpp_selftest_scan_pipe_timeout(const int32_t *in, int32_t *out, int64_t length,

@@ -16,13 +16,9 @@ namespace edpp {
 // class recorded for that primitive and element size, else `fallback`.
 int tuned_variant(int prim, int elem_bytes, int64_t length, int fallback);
 
-// The variant of that entry if edpp_tune_set recorded it, else -1: a choice
-// that goes before the rules by which a scan of moderate size leaves the table.
-int chosen_variant(int prim, int elem_bytes, int64_t length);
-
 // Scan of `length` elements of `elem_bytes` bytes (4: int32, 8: int64) with
-// an explicit variant of `algo` (EDPP_SCAN_LOOKBACK: tile shape, EDPP_SCAN_RTS:
-// slice length of the chunked form), for the autotuner.  Same arguments and
+// an explicit variant of `algo` (0: the default form of the length, else a
+// look-back tile shape or a slice length of the chunked form), for the autotuner.  Same arguments and
 // results as edpp_scan_exclusive_i32 / _i64.
 int scan_with_variant(const void *in, void *out, int64_t length, int elem_bytes, int algo,
                       int variant, void *ws, size_t ws_bytes, void *stream);

@@ -483,15 +483,17 @@ void edpp_server_destroy(edpp_server *server);
  * recorded class, else the default (variant 0).  The reference fixes its
  * tunables per device by hand (R, L, local and grid sizes of scan_chained,
  * opencl/test/test_scan_global.cpp:87-94); here they are measured.
- *   EDPP_TUNE_SCAN_LOOKBACK  look-back tile shape (threads x 16-byte chunks):
- *                            0 128x8 (16 KB), 1 256x8 (32 KB), 2 512x4 (32 KB);
- *                            3 the pipelined one-launch scan (variant 1 for
- *                            arrays off 16-byte alignment)
- *   EDPP_TUNE_SCAN_RTS       0 the pipelined one-launch scan (arrays off 16-byte
- *                            alignment: slices of two tiles); else the slice
- *                            of the chunked reduce-then-scan (inputs larger
- *                            than 60% of L2): 1 one tile, 2 four, 3 two with
- *                            L2 eviction hints (first read kept, second read
+ *   Scans, variant 0         the form of the length: one thread-block cluster up
+ *                            to 256 KB, two launches up to 48 MB (64-bit elements
+ *                            32 MB), beyond that the pipelined one-launch scan
+ *                            (arrays off 16-byte alignment: look-back variant 1,
+ *                            slices of the chunked reduce-then-scan)
+ *   EDPP_TUNE_SCAN_LOOKBACK  tile shape (threads x 16-byte chunks): 1 256x8, 2
+ *                            512x4 (32 KB each); 3 the pipelined one-launch scan
+ *                            (variant 1 for arrays off 16-byte alignment)
+ *   EDPP_TUNE_SCAN_RTS       slice of the chunked reduce-then-scan (inputs larger
+ *                            than 60% of L2): 1 one tile, 2 four, 3 two with L2
+ *                            eviction hints (first read kept, second read
  *                            demoted), 4 two tiles and the chunked form also
  *                            below 60% of L2
  *   EDPP_TUNE_GATHER         0 tiled form, 1 direct single sweep (the choice
@@ -507,10 +509,7 @@ typedef enum {
 
 /* Number of variants of a primitive (0: not tunable). */
 int edpp_tune_variants(int primitive);
-/* Record `variant` (measured at `ms`, informational) for the class.  Look-back
- * and reduce-then-scan calls of up to 256 KB (one thread-block cluster) and 48
- * MB (64-bit elements: 32 MB; two launches), which otherwise run in those forms
- * whatever the table holds, take a variant set here. */
+/* Record `variant` (measured at `ms`, informational) for the class. */
 int edpp_tune_set(int primitive, int elem_bytes, int log2_length, int variant, float ms);
 /* The variant a call of `length` elements takes now (EDPP_OK), or the
  * default with EDPP_EINVAL when the table has no entry for the primitive. */
