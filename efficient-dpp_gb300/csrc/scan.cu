@@ -1016,7 +1016,12 @@ int scan_impl(const T *in, T *out, int64_t n, int algo, void *ws, size_t ws_byte
   }
   if (algo == EDPP_SCAN_RTS) {
     // larger than L2: the chunked one-launch form, which reads each element
-    // from DRAM once
+    // from DRAM once.  With only the output off 16-byte alignment its stores are
+    // the slow part, and slices of four tiles are ahead from 256 MB on: two / four
+    // tiles, int32 2^25 72.2 / 80.3 us, 2^26 142 / 138, 2^28 564 / 537; int64 2^24
+    // 72.1 / 80.3, 2^25 143 / 135, 2^28 1134 / 1008.
+    if (variant == 0 && tma && !vec_out && n >= (256ll << 20) / static_cast<int64_t>(sizeof(T)))
+      variant = 2;
     int s;
     switch (variant) {
       case 3:

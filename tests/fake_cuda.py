@@ -42,14 +42,14 @@ class Fake:
         self.lib.fake_log.restype = ctypes.c_char_p
 
     def launches(self, call, refuse=0, blocks_per_sm=2):
-        """(status, [(kernel, blocks, kind)]) of call(lib)."""
+        """(status, [(kernel, blocks, kind, its mangled template arguments)]) of call(lib)."""
         self.lib.fake_reset(refuse, blocks_per_sm)
         status = call(self.lib)
         out = []
         for line in self.lib.fake_log().decode().splitlines():
             name, blocks, kind = line.split()
             kernel, = (k for k in KERNELS if f"{len(k)}{k}" in name)  # of the mangled name
-            out.append([kernel, int(blocks), int(kind)])
+            out.append([kernel, int(blocks), int(kind), name.split(kernel, 1)[1]])
         return status, out
 
 

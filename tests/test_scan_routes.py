@@ -106,6 +106,20 @@ def test_workspace_off_16_bytes(fake_lib):
 result = [[n, algo] + fake.launches(lambda l: l.edpp_scan_exclusive_i32(IN, OUT, n, algo, WS + 8, BIG, None))[1][-1:]
           for n in (100_000, 1 << 19, (1 << 19) + 1, 1 << 23, 1 << 25) for algo in (0, 1)]
 """)
-    for n, algo, (kernel, _, _) in got:
+    for n, algo, (kernel, *_) in got:
         small = "scan_lookback_kernel" if algo == 0 else "rts_fused_kernel"
         assert kernel == (small if n <= 1 << 19 else "scan_pipe_kernel"), (n, algo)
+
+
+@pytest.mark.parametrize("t,elem", [("i32", 4), ("f32", 4), ("i64", 8)])
+def test_slices_of_unaligned_reduce_then_scan(fake_lib, t, elem):
+    """Slices of four tiles from 256 MB on where only the output is off 16 bytes."""
+    line = (256 << 20) // elem
+    got = fake_cuda.run(fake_lib, f"""
+result = [fake.launches(lambda l: l.edpp_scan_exclusive_{t}(IN + i * {elem}, OUT + o * {elem}, n, 1, WS, BIG, None))
+          for n in ({line} - 1, {line}, 4 * {line} + 3) for i, o in ((1, 0), (0, 1), (1, 1))]
+""")
+    for k, (status, kernels) in enumerate(got):
+        assert status == 0 and [x[0] for x in kernels] == ["rts_chunked_kernel"]
+        four = k % 3 == 1 and k > 3
+        assert ("ELi4E" if four else "ELi2E") in kernels[0][3], (k, kernels)
