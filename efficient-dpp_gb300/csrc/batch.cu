@@ -679,11 +679,20 @@ __global__ void __launch_bounds__(kThreads, 4)
 namespace {
 
 // Scan tiles from which the pipelined scan runs.  It costs some 6 us more to
-// launch (cooperatively, after the kernels before it have drained) and 2.5 ns
-// less per tile: batches of 512 segments, 1.7e7 elements (1360 scan tiles) 92 us
-// without and 97 with it, 6.7e7 elements (5400) 257 and 246; 4096 segments of
-// 6.7e7 elements even, of 2.7e8 881 and 847.
+// launch (cooperatively, after the kernels before it have drained): mixed batches
+// of 512 segments, 1.7e7 elements (1360 scan tiles) 92 us without and 97 with it,
+// 6.7e7 elements (5400) 257 and 246.
 constexpr int64_t kPipeTiles = 4096;
+
+// What the pipelined scan gains on a segment of `tiles` tiles over one block per
+// tile, in half nanoseconds.  Its tiles take 5.2 ns each, short or full.  Those of
+// the look-back take longer the longer their segment's chain: scans of 2^28 elements
+// in equal segments, us per launch, look-back / pipelined: 1 tile 317 / 350, 4 tiles
+// 331 / 346, 8 344 / 344, 16 380 / 342, 32 446 / 339, 64 490 / 339, 4096 563 / 337;
+// 65536 segments shorter than a tile 204 / 313.
+int64_t pipe_gain(int64_t tiles) {
+  return tiles < 8 ? -tiles : tiles < 16 ? 0 : tiles < 32 ? tiles : 3 * tiles;
+}
 constexpr size_t kHdrB = 256;  // ticket (u64) + abort flag (u32)
 
 int build_plan(const edpp_segment *in, int num, const edpp_batch_tuning *tune, BatchPlanImpl &p) {
@@ -702,6 +711,8 @@ int build_plan(const edpp_segment *in, int num, const edpp_batch_tuning *tune, B
                      [&](int a, int b) { return in[a].length > in[b].length; });
   // state: scan tile words first (zeroed per launch), then split histograms
   size_t scan_state = 0, split_state = 0;
+  bool scan_aligned = true;  // every scan segment starts on a multiple of 4 elements
+  int64_t gain = 0;
   for (int i = 0; i < num; ++i) {
     const edpp_segment &s = in[i];
     if (s.length < 0 || s.offset < 0) return EDPP_EINVAL;
@@ -718,7 +729,8 @@ int build_plan(const edpp_segment *in, int num, const edpp_batch_tuning *tune, B
     d.buckets = s.op == EDPP_BATCH_SPLIT ? s.buckets : 0;
     if (s.op == EDPP_BATCH_SCAN) {
       d.state = static_cast<int64_t>(scan_state);
-      p.scan_aligned = p.scan_aligned && (s.offset & 3) == 0;
+      scan_aligned = scan_aligned && (s.offset & 3) == 0;
+      gain += pipe_gain(d.tiles);
       scan_state += LookbackState<int32_t>::bytes(d.tiles);
     }
     p.segs[static_cast<size_t>(i)] = d;
@@ -784,6 +796,7 @@ int build_plan(const edpp_segment *in, int num, const edpp_batch_tuning *tune, B
     p.n_scan = static_cast<int64_t>(scan.size());
     p.n_gather = static_cast<int64_t>(gather.size());
     p.n_split = static_cast<int64_t>(split.size());
+    p.scan_pipe = p.n_scan >= kPipeTiles && scan_aligned && gain > 0;
     p.tasks = std::move(scan);
     p.tasks.insert(p.tasks.end(), gather.begin(), gather.end());
     p.tasks.insert(p.tasks.end(), split.begin(), split.end());
@@ -884,10 +897,10 @@ int edpp_batch_launch(const edpp_batch_plan *plan, const int32_t *in0, const int
                   reinterpret_cast<unsigned *>(w + 8), aligned16(in0), aligned16(in1),
                   p.num_segs};
   if (p.schedule == EDPP_BATCH_SCHEDULE_KINDS) {
-    // Many scan tiles: the pipelined scan (scan_pipe.cu).  4096 segments all
-    // scan, 2^30 elements: 2.00 -> 1.31 ms.
+    // Many scan tiles in long segments: the pipelined scan (scan_pipe.cu).  4096
+    // segments all scan, 2^30 elements: 2.00 -> 1.31 ms.
     bool scanned = p.n_scan == 0;
-    if (!scanned && p.n_scan >= kPipeTiles && p.scan_aligned && aligned16(in0) && aligned16(out0)) {
+    if (!scanned && p.scan_pipe && aligned16(in0) && aligned16(out0)) {
       const int s = scan_pipe_tasks(in0, out0, dsegs, dtasks, p.num_segs, p.n_scan, w + p.off_state,
                                     reinterpret_cast<unsigned *>(w + 8), st, kDefaultWaitNs, fault);
       if (s != EDPP_OK && s != EDPP_ENOMEM) return s;

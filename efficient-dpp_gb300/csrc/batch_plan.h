@@ -49,7 +49,7 @@ struct BatchPlanImpl {
   int num_segs = 0;
   int blocks_per_sm = 4;
   int schedule = 0;  // edpp_batch_schedule
-  bool scan_aligned = true;  // every scan segment starts on a multiple of 4 elements
+  bool scan_pipe = false;  // the scan tiles run in the pipelined kernel (aligned arrays)
   int64_t total_elems = 0;
 };
 
