@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(kIndexThreads, index_blocks<LAYOUT, TILE, kFus
                        int64_t n, int buckets, int shift, int64_t tiles,
                        const int32_t *__restrict__ his, bool tma, bool exact, uint64_t timeout_ns,
                        unsigned *fault, FusedArgs fused) {
-  using C = PosStage<kIndexThreads, TILE>;
+  using C = PosStage<kIndexThreads, TILE, !kFused && TILE == 8192>;
   constexpr int THREADS = kIndexThreads;
   extern __shared__ __align__(128) unsigned char smem[];
   int32_t *s_keys = reinterpret_cast<int32_t *>(smem);
