@@ -309,7 +309,8 @@ __device__ __forceinline__ uint32_t load_split_tile(int64_t gbase, int count, co
 // bucket in between.  Bound by the shared-memory pipe.  4096 segments, 2^30
 // elements, 64 buckets, all split 4.74 -> 4.10 ms against per-warp lane masks
 // with the pairs re-laid out; four blocks per SM (three: 4.60, five: 4.16; 512
-// threads, four blocks: 4.33).
+// threads, four blocks: 4.33).  UNROLL: steps of the write-out in flight.
+template <int UNROLL>
 __device__ __forceinline__ void split_tile_index(const DevSeg &seg, int tile, const TaskIO &io,
                                                  BatchSmem &sm, uint64_t *bar, uint32_t &phase) {
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
@@ -371,7 +372,7 @@ __device__ __forceinline__ void split_tile_index(const DevSeg &seg, int tile, co
     io.out0[o] = e.x;
     io.out1[o] = e.y;
   };
-  if (__syncthreads_or(P::write_out<4>(sm.split.pos, count, load, bucket_of, store))) {
+  if (__syncthreads_or(P::write_out<UNROLL>(sm.split.pos, count, load, bucket_of, store))) {
     P::place_exact(sm.split.cnt16, B, count, bucket_at, sm.split.pos);
     __syncthreads();
     P::write_out<1>(sm.split.pos, count, load, bucket_of, store);
@@ -471,14 +472,23 @@ __device__ __forceinline__ void split_tile_votes(const DevSeg &seg, int tile, co
 }
 
 // Form chosen once per tile, so each form's unrolled loop is compiled on its own.
+template <int UNROLL>
 __device__ __forceinline__ void split_tile_task(const DevSeg &seg, int tile, const TaskIO &io,
                                                 BatchSmem &sm, uint64_t *bar, uint32_t &phase) {
-  if (seg.buckets > 8) split_tile_index(seg, tile, io, sm, bar, phase);
+  if (seg.buckets > 8) split_tile_index<UNROLL>(seg, tile, io, sm, bar, phase);
   else split_tile_votes(seg, tile, io, sm, bar, phase);
 }
 
 // ---- QUEUE schedule: one persistent launch over the work queue ----
-__global__ void __launch_bounds__(kThreads, 3)
+// Bound by the latency of a tile: a block runs its tasks one after another.  So four
+// blocks per SM (64 registers, a few spilled) where the plan asks for as many, and the
+// whole write-out of a split tile in flight.  4096 segments, 2^28 elements, three
+// blocks and four steps in flight against this, ms: all scan 0.889 and 0.722, all split
+// 16 buckets 2.71 and 2.14 (per-warp lane masks 2.57), 64 buckets 2.76 and 2.19, mixed
+// 1.52 and 1.22.  Gathers alone live off L1, which the fourth block's shared memory
+// takes: 300 segments of 3.4e7 elements 180 and 196 us, so they stay with three.
+template <int BLOCKS>
+__global__ void __launch_bounds__(kThreads, BLOCKS)
     batch_kernel(const DevSeg *__restrict__ segs, const DevTask *__restrict__ tasks, int num_tasks,
                  TaskIO io, Ctrl *ctrl, unsigned long long *ticket) {
   __shared__ BatchSmem sm;
@@ -560,7 +570,7 @@ __global__ void __launch_bounds__(kThreads, 3)
         take_next();
       }
       __syncthreads();
-      if (s_flag) split_tile_task(seg, task.tile, io, sm, &bar, phase);
+      if (s_flag) split_tile_task<16>(seg, task.tile, io, sm, &bar, phase);
     }
     // this task's generic accesses of shared memory before the next task's
     // bulk copies into it; shared memory and s_task reused by the next task
@@ -670,7 +680,7 @@ __global__ void __launch_bounds__(kThreads, 4)
   wait_dependencies();
   DevSeg seg;
   uint32_t phase = 0;
-  if (task_in_plan(task, segs, io, seg)) split_tile_task(seg, task.tile, io, sm, &bar, phase);
+  if (task_in_plan(task, segs, io, seg)) split_tile_task<4>(seg, task.tile, io, sm, &bar, phase);
 }
 
 }  // namespace
@@ -733,6 +743,7 @@ int build_plan(const edpp_segment *in, int num, const edpp_batch_tuning *tune, B
       gain += pipe_gain(d.tiles);
       scan_state += LookbackState<int32_t>::bytes(d.tiles);
     }
+    if (s.op != EDPP_BATCH_GATHER) p.gathers_only = false;
     p.segs[static_cast<size_t>(i)] = d;
     p.total_elems += s.length;
   }
@@ -931,22 +942,24 @@ int edpp_batch_launch(const edpp_batch_plan *plan, const int32_t *in0, const int
     if (s == EDPP_OK && p.n_split) s = launch(kind_split_kernel, p.n_split, dsegs, split_tasks, io);
     return s;
   }
-  static std::once_flag occ_once[64];
-  static cudaError_t occ_err[64];
-  static int resident[64];
+  const int k = p.blocks_per_sm >= 4 && !p.gathers_only;
+  const auto kernel = k ? batch_kernel<4> : batch_kernel<3>;
+  static std::once_flag occ_once[2][64];
+  static cudaError_t occ_err[2][64];
+  static int resident[2][64];
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) dev = 0;
-  std::call_once(occ_once[dev], [dev] {
-    occ_err[dev] = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident[dev], batch_kernel,
-                                                                 kThreads, 0);
+  std::call_once(occ_once[k][dev], [=] {
+    occ_err[k][dev] =
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident[k][dev], kernel, kThreads, 0);
   });
-  if (occ_err[dev] != cudaSuccess) return EDPP_ECUDA;
+  if (occ_err[k][dev] != cudaSuccess) return EDPP_ECUDA;
   // blocks beyond what stays resident would only start once the queue is empty
-  const int per_sm = std::max(1, std::min(p.blocks_per_sm, resident[dev]));
+  const int per_sm = std::max(1, std::min(p.blocks_per_sm, resident[k][dev]));
   int64_t blocks = static_cast<int64_t>(device_sm_count()) * per_sm;
   blocks = min64(blocks, static_cast<int64_t>(p.tasks.size()));
-  batch_kernel<<<static_cast<unsigned>(max64(blocks, 1)), kThreads, 0, st>>>(
+  kernel<<<static_cast<unsigned>(max64(blocks, 1)), kThreads, 0, st>>>(
       dsegs, dtasks, static_cast<int>(p.tasks.size()), io,
       reinterpret_cast<Ctrl *>(w + p.off_ctrl), reinterpret_cast<unsigned long long *>(w));
   return launch_status();

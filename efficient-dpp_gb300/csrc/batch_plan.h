@@ -49,6 +49,7 @@ struct BatchPlanImpl {
   int num_segs = 0;
   int blocks_per_sm = 4;
   int schedule = 0;  // edpp_batch_schedule
+  bool gathers_only = true;
   bool scan_pipe = false;  // the scan tiles run in the pipelined kernel (aligned arrays)
   int64_t total_elems = 0;
 };

@@ -48,3 +48,23 @@ for shift in (0, 2):
     for k, (status, kernels) in enumerate(got):
         want = "scan_pipe_kernel" if pipe and k == 0 else "kind_scan_kernel"  # aligned, not moved
         assert status == 0 and [x[0] for x in kernels] == [want], k
+
+
+@pytest.mark.parametrize("ops,asked,blocks", [([0], 0, 4), ([1], 4, 4), ([0, 1, 2], 0, 4), ([2], 0, 3),
+                                              ([2, 2], 4, 3), ([1], 3, 3), ([1], 1, 1), ([0, 2], 8, 4)])
+def test_queue_blocks_per_sm(fake_lib, ops, asked, blocks):
+    """The work-queue kernel: four blocks per SM where asked for, three for gathers alone."""
+    status, kernels = fake_cuda.run(fake_lib, f"""
+import ctypes
+import numpy as np
+from edpp.batch import SEG_DTYPE, Tuning
+segs = np.zeros(len({ops}), SEG_DTYPE)
+segs["length"], segs["op"], segs["buckets"] = 1 << 22, {ops}, 16
+segs["offset"] = np.arange(len(segs), dtype=np.int64) << 22
+plan, tuning = ctypes.c_void_p(), Tuning({asked}, 1, 1, 1)
+assert fake.lib.edpp_batch_plan_create(segs.ctypes.data, len(segs), ctypes.byref(tuning), ctypes.byref(plan)) == 0
+result = fake.launches(lambda l: l.edpp_batch_launch(plan, IN, IN1, OUT, OUT1, WS, BIG, None), 0, {max(blocks, 3)})  # what fits of each kernel
+""")
+    assert status == 0 and len(kernels) == 1
+    assert kernels[0][0] == "batch_kernel" and kernels[0][1] == 152 * blocks
+    assert f"Li{4 if blocks == 4 else 3}E" in kernels[0][3]
