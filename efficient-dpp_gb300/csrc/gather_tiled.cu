@@ -20,6 +20,9 @@
 //   restore  one block per tile: out[i] = the tile's value at slots[i], read
 //            at random from shared memory
 //
+// A tile whose requests lie close together is gathered by the group kernel itself,
+// with empty runs for the others (see kNear).
+//
 // Nothing is counted or claimed globally and the values need no second
 // grouping on the way back, since a tile's values never leave the tile:
 // 32 bytes per element (group 4 + 6, fetch 4 + 4 + 4, restore 6 + 4), against
@@ -43,6 +46,18 @@ constexpr uint32_t kNoSlot = 0xffffu;   // an index outside [0, n): out[i] keeps
 constexpr int kFetchThreads = 256;
 constexpr int kFetchRuns = 4;           // tiles per warp
 constexpr int kFetchTiles = kFetchThreads / 32 * kFetchRuns;
+
+// A tile is read directly if its requests span at most kNear elements (one 32-byte
+// sector per request: from DRAM that costs no more than the tiled way), if three
+// quarters of its vectors lie within a 128-byte line each, or, in a large array, if the
+// tile and one request of every 16th tile around it span at most kNearAll (a quarter of
+// L2, for all tiles in flight): grouping gains nothing there.  2^26 requests, us, direct
+// sweep / all tiles grouped / so: identity 129 / 673 / 170, rows of 4096 in random order
+// 131 / 634 / 172, random within 4 MB 263 / 888 / 337, one address 90 / 922 / 119; a
+// random permutation 999 / 524 / 524.  (The rest over the direct sweep is the other two
+// kernels finding nothing to do.  A transpose, 275 / 683 / 700, looks random to a tile.)
+constexpr uint32_t kNear = 8 * kTile, kNearAll = 1u << 23;
+constexpr int64_t kNearAllFrom = 1 << 24;  // requests
 
 // Windows of 2^log_w elements: 64 of them (runs of 128 requests, 512 bytes)
 // while they fit L2 comfortably, then more windows up to kMaxWin, then larger
@@ -84,12 +99,16 @@ GatherLayout gather_layout(const GatherPlan &p) {
 __global__ void __launch_bounds__(kThreads, 3)
     gather_group_kernel(const int32_t *__restrict__ loc, int64_t n, int log_w, int nwin,
                         int64_t stride, int32_t *__restrict__ buf, uint16_t *__restrict__ slots,
-                        uint16_t *__restrict__ offs, bool vec) {
+                        uint16_t *__restrict__ offs, bool vec, const int32_t *__restrict__ in,
+                        int32_t *__restrict__ out, bool vec_out, bool near) {
   __shared__ alignas(16) int32_t stage[kTile];
   __shared__ uint32_t scnt[kMaxWin], soff[kMaxWin];
   __shared__ uint32_t s_total;
-  const int t = threadIdx.x;
+  __shared__ uint32_t s_lo[kThreads / 32], s_hi[kThreads / 32], s_tight[kThreads / 32];
+  __shared__ bool s_maybe;
+  const int t = threadIdx.x, lane = t & 31;
   const int64_t tile = blockIdx.x, base = tile * kTile;
+  const uint32_t un = static_cast<uint32_t>(n);
   if (t < kMaxWin) scnt[t] = 0;
   if (tile + 1 == gridDim.x) {  // the rows of offs end in empty runs
     const int pad = static_cast<int>(stride - tile - 1);
@@ -111,8 +130,71 @@ __global__ void __launch_bounds__(kThreads, 3)
     }
     l[4 * k] = q.x, l[4 * k + 1] = q.y, l[4 * k + 2] = q.z, l[4 * k + 3] = q.w;
   }
+  // How near its requests lie: the first warp's first vectors tell a random tile apart,
+  // all of them decide.
+  uint32_t lo = ~0u, hi = 0, tight = 0;
+  auto widen = [&](int k) {  // by a vector; tight: vectors whose requests lie within a line
+    uint32_t a = ~0u, b = 0;
+#pragma unroll
+    for (int e = 4 * k; e < 4 * k + 4; ++e) {
+      const uint32_t u = static_cast<uint32_t>(l[e]);
+      if (u < un) a = min(a, u), b = max(b, u);
+    }
+    lo = min(lo, a), hi = max(hi, b);
+    tight += __popc(__ballot_sync(0xffffffffu, b < a + 32 || b < a));
+  };
+  auto join = [&](uint32_t a, uint32_t b) {
+    lo = __reduce_min_sync(0xffffffffu, a);
+    hi = __reduce_max_sync(0xffffffffu, b);
+  };
+  const uint32_t near_all = n > kNearAllFrom ? kNearAll : kNear;
+  if (t < 32) {
+    widen(0);
+    join(lo, hi);
+    if (t == 0) s_maybe = near && (tight >= 16 || hi < lo || hi - lo < near_all);
+  }
   __syncthreads();
-  const uint32_t un = static_cast<uint32_t>(n);
+  if (s_maybe) {
+    tight = 0;
+#pragma unroll
+    for (int k = 0; k < kPer / 4; ++k) widen(k);
+    join(lo, hi);
+    if (lane == 0) s_lo[t >> 5] = lo, s_hi[t >> 5] = hi, s_tight[t >> 5] = tight;
+    __syncthreads();
+    constexpr int kWarps = kThreads / 32;
+    join(s_lo[lane & (kWarps - 1)], s_hi[lane & (kWarps - 1)]);
+    tight = __reduce_add_sync(0xffffffffu, lane < kWarps ? s_tight[lane] : 0u);
+    bool direct = tight >= kThreads / 4 * 3 * (kPer / 4) || hi < lo || hi - lo < kNear;
+    if (!direct && n > kNearAllFrom) {
+      const int64_t j = base + (lane - 16) * (16ll * kTile) + 64 * lane;
+      const uint32_t u = static_cast<uint32_t>(j >= 0 && j < n ? loc[j] : -1);
+      join(u < un ? min(lo, u) : lo, u < un ? max(hi, u) : hi);
+      direct = hi - lo < kNearAll;
+    }
+    if (direct) {
+      for (int w = t; w <= nwin; w += kThreads) offs[w * stride + tile] = 0;
+#pragma unroll
+      for (int k = 0; k < kPer / 4; ++k) {
+        const int64_t i = base + (k * kThreads + t) * 4;
+        int32_t v[4];
+        bool all = vec_out;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const bool ok = static_cast<uint32_t>(l[4 * k + q]) < un;
+          all = all && ok;
+          v[q] = ok ? in[l[4 * k + q]] : 0;
+        }
+        if (all) {
+          __stcs(reinterpret_cast<int4 *>(out + i), make_int4(v[0], v[1], v[2], v[3]));
+        } else {
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            if (static_cast<uint32_t>(l[4 * k + q]) < un) out[i + q] = v[q];
+        }
+      }
+      return;
+    }
+  }
   uint32_t rk[kPer / 2];  // two 16-bit ranks per register
 #pragma unroll
   for (int e = 0; e < kPer; ++e) {
@@ -272,8 +354,12 @@ int gather_tiled(const int32_t *in, int32_t *out, int64_t n, const int32_t *loc,
   auto *slots = reinterpret_cast<uint16_t *>(w + L.slots);
   auto *offs = reinterpret_cast<uint16_t *>(w + L.offs);
   const unsigned tiles = static_cast<unsigned>(p.tiles);
+  // a tile read directly is written while others still read: not in place
+  auto apart = [n](const int32_t *a, const int32_t *b) { return a + n <= b || b + n <= a; };
+  const bool near = apart(in, out) && apart(loc, out);
   gather_group_kernel<<<tiles, kThreads, 0, st>>>(loc, n, p.log_w, p.nwin, p.stride, buf, slots,
-                                                  offs, aligned16(loc));
+                                                  offs, aligned16(loc), in, out, aligned16(out),
+                                                  near);
   const unsigned groups = static_cast<unsigned>(p.stride / kFetchTiles);
   gather_fetch_kernel<<<static_cast<unsigned>(p.nwin) * groups, kFetchThreads, 0, st>>>(
       in, p.stride, groups, offs, buf);

@@ -140,7 +140,8 @@ int edpp_scatter_i32_ws(const int32_t *in, int32_t *out, int64_t length,
 /* Tiled gather / scatter: the same results again, for every pass count
  * (pass >= 0 is accepted for the same signature; the windows are fixed by
  * L2 and shared memory).  The gather groups its requests by L2-sized window
- * inside tiles of 8192 and reads each window while it sits in L2.  The
+ * inside tiles of 8192 and reads each window while it sits in L2 (tiles whose
+ * requests lie close together are read directly); in, loc and out may overlap.  The
  * scatter partitions its pairs twice by window (128 coarse windows, then
  * fine windows of 2^14 or 2^15 elements) and one block per fine window
  * serves them inside a shared-memory copy of that window; above 2^29
