@@ -67,8 +67,9 @@ double split_any(const int *d_in, int *d_out, int *d_start, int length, int buck
 
 }  // namespace
 
-// Multi-pass gather / scatter through the shared-memory-window form: the same
-// results as the reference's pass-by-pass sweeps for every pass count.
+// Multi-pass gather / scatter through the tiled forms, or a direct sweep while the
+// randomly accessed array stays in L2: the same results as the reference's
+// pass-by-pass sweeps for every pass count.
 double gather(const int *d_in, int *d_out, int length, const int *d_loc, int, int, int pass) {
   if (pass < 1) return -1;
   if (edpp_gather_prefers_direct(length))  // the source stays in L2: one direct sweep
@@ -82,7 +83,10 @@ double gather(const int *d_in, int *d_out, int length, const int *d_loc, int, in
 
 double scatter(const int *d_in, int *d_out, int length, const int *d_loc, int, int, int pass) {
   if (pass < 1) return -1;
-  if (edpp_scatter_prefers_direct(length))  // the destination stays in L2
+  // The destination stays in L2: one direct sweep, which writes while it reads, so not
+  // over d_in or d_loc (the tiled form reads all of both first).
+  auto apart = [&](const int *a) { return a + length <= d_out || d_out + length <= a; };
+  if (edpp_scatter_prefers_direct(length) && apart(d_in) && apart(d_loc))
     return timed([&] { return edpp_scatter_i32(d_in, d_out, length, d_loc, 1, nullptr); });
   Temp ws(edpp_scatter_tiled_workspace_size(length));
   if (!ws.ok()) return -1;

@@ -234,14 +234,18 @@ def _gs(kind, inp, loc, passes, out, method, ws):
     if out is None:
         out = torch.zeros(n, dtype=torch.int32, device=loc.device)
     st = _stream()
+    src, dst, idx = _p(inp), _p(out), _p(loc)
     if method == "auto":  # the faster schedule for this size
-        direct = (lib().edpp_gather_prefers_direct if kind == "gather"
-                  else lib().edpp_scatter_prefers_direct)
-        method = "sweep" if direct(n) else "tiled"
+        if kind == "gather":
+            direct = lib().edpp_gather_prefers_direct(n)
+        else:  # a sweep writes while it reads; the tiled scatter reads inp and loc first
+            direct = (abs(src - dst) >= 4 * n and abs(idx - dst) >= 4 * n
+                      and lib().edpp_scatter_prefers_direct(n))
+        method = "sweep" if direct else "tiled"
         passes = 1 if method == "sweep" else passes
     if method == "sweep":
         f = lib().edpp_gather_i32 if kind == "gather" else lib().edpp_scatter_i32
-        check(f(_p(inp), _p(out), n, _p(loc), int(passes), st), kind)
+        check(f(src, dst, n, idx, int(passes), st), kind)
     elif method in ("partition", "tiled"):
         if ws is None:
             ws = workspace(gs_workspace_bytes(kind, n, passes, method), loc.device)
@@ -249,7 +253,7 @@ def _gs(kind, inp, loc, passes, out, method, ws):
             f = lib().edpp_gather_i32_ws if kind == "gather" else lib().edpp_scatter_i32_ws
         else:
             f = lib().edpp_gather_i32_tiled if kind == "gather" else lib().edpp_scatter_i32_tiled
-        check(f(_p(inp), _p(out), n, _p(loc), int(passes), _p(ws), ws.numel(), st), kind)
+        check(f(src, dst, n, idx, int(passes), _p(ws), ws.numel(), st), kind)
     else:
         raise ValueError(method)
     return out

@@ -141,7 +141,7 @@ int edpp_scatter_i32_ws(const int32_t *in, int32_t *out, int64_t length,
  * (pass >= 0 is accepted for the same signature; the windows are fixed by
  * L2 and shared memory).  The gather groups its requests by L2-sized window
  * inside tiles of 8192 and reads each window while it sits in L2 (tiles whose
- * requests lie close together are read directly); in, loc and out may overlap.  The
+ * requests lie close together are read directly).  The
  * scatter partitions its pairs twice by window (128 coarse windows, then
  * fine windows of 2^14 or 2^15 elements) and one block per fine window
  * serves them inside a shared-memory copy of that window; above 2^29
@@ -159,7 +159,9 @@ int edpp_scatter_i32_tiled(const int32_t *in, int32_t *out, int64_t length,
  * single sweep (edpp_gather_i32 / edpp_scatter_i32, pass 1) than in the tiled
  * form on the current device.  Gather: the tuning table's choice for this
  * size class when it has one (EDPP_TUNE_GATHER), else whether the source fits
- * L2.  Scatter: whether the destination fits 80% of L2. */
+ * L2.  Scatter: whether the destination fits 80% of L2.  A direct sweep writes
+ * while it reads, so its arrays must not overlap; the tiled forms read in and
+ * loc before the first write. */
 int edpp_gather_prefers_direct(int64_t length);
 int edpp_scatter_prefers_direct(int64_t length);
 

@@ -115,26 +115,39 @@ cudaError_t cudaMemcpyAsync(void *, const void *, size_t, cudaMemcpyKind, cudaSt
 }
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
 
+cudaError_t cudaStreamQuery(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaEventCreate(cudaEvent_t *e) {
+  *e = nullptr;
+  return cudaSuccess;
+}
+cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaEventElapsedTime(float *ms, cudaEvent_t, cudaEvent_t) {
+  *ms = 1;
+  return cudaSuccess;
+}
+cudaError_t cudaMallocAsync(void **p, size_t, cudaStream_t) {
+  *p = g_symbol;
+  return cudaSuccess;
+}
+cudaError_t cudaFreeAsync(void *, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaMemcpyFromSymbol(void *dst, const void *, size_t n, size_t, cudaMemcpyKind) {
+  std::memset(dst, 0, n);
+  return cudaSuccess;
+}
+
 // Never called by what is tested here.
 #define UNUSED(name, ...) \
   cudaError_t name(__VA_ARGS__) { return cudaErrorNotSupported; }
 UNUSED(cudaDeviceSynchronize)
-UNUSED(cudaEventCreate, cudaEvent_t *)
-UNUSED(cudaEventDestroy, cudaEvent_t)
-UNUSED(cudaEventElapsedTime, float *, cudaEvent_t, cudaEvent_t)
-UNUSED(cudaEventRecord, cudaEvent_t, cudaStream_t)
 UNUSED(cudaFree, void *)
-UNUSED(cudaFreeAsync, void *, cudaStream_t)
 UNUSED(cudaFreeHost, void *)
 UNUSED(cudaLaunchHostFunc, cudaStream_t, cudaHostFn_t, void *)
 UNUSED(cudaMalloc, void **, size_t)
-UNUSED(cudaMallocAsync, void **, size_t, cudaStream_t)
 UNUSED(cudaMallocHost, void **, size_t)
-UNUSED(cudaMemcpyFromSymbol, void *, const void *, size_t, size_t, cudaMemcpyKind)
 UNUSED(cudaMemcpyToSymbol, const void *, const void *, size_t, size_t, cudaMemcpyKind)
 UNUSED(cudaSetDevice, int)
 UNUSED(cudaStreamCreateWithFlags, cudaStream_t *, unsigned)
 UNUSED(cudaStreamDestroy, cudaStream_t)
-UNUSED(cudaStreamQuery, cudaStream_t)
 
 }  // extern "C"
