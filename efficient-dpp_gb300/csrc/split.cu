@@ -24,11 +24,11 @@
 //              on, depending on the layout, one atomic per element ranks and
 //              only source positions are re-laid out (split_index.cuh).
 //
-// Inputs whose tiles are all resident at once (up to 2.4 million elements) take
-// one cooperative launch instead (the fused form of the scatter kernel): the
-// tile is read once, its counts come from its ranking, and the blocks exchange
-// them through his.  With few tiles times buckets they take two plain launches:
-// the counts, then that kernel, which adds them up itself.
+// Inputs whose tiles are all resident at once (up to 2.4 million elements) add up
+// the tiles' counts in the scatter kernel itself (its fused form).  With few tiles
+// times buckets they take two plain launches: the counts, then that kernel.  With
+// more, and position staging, one cooperative launch: the tile is read once, its
+// counts come from its ranking, and the blocks exchange them through his.
 //
 // Ranks follow input order inside a warp segment, warp segments follow
 // input order inside a tile, tiles follow input order in the scan: the split
@@ -174,17 +174,18 @@ size_t scatter_smem_bytes(int buckets, bool bulk = false) {
 // Two blocks per SM (their staging fills shared memory): at most 64 registers.
 // For fewer than index_buckets() buckets.
 //
-// kFused: the whole split in one cooperative launch, for inputs whose tiles are
-// all resident together.  The tile's bucket counts come from its own ranking;
-// they are published as row t of his, and once every block has arrived at
-// *fused.arrived (bounded wait) each block adds up what precedes its runs: the
-// smaller buckets' totals and its bucket's counts in the tiles before.  The
-// tile waits in registers meanwhile.
+// kFused, for inputs whose tiles are all resident together: each block adds up what
+// precedes its runs, the smaller buckets' totals and its bucket's counts in the tiles
+// before, from his, one row per tile; the tile waits in registers (here) or in shared
+// memory (split_index.cuh).
 //
-// Where few words are exchanged, the counts come from split_counts_kernel instead
-// (arrived null): two plain launches, no memset and no waiting among blocks.  The
-// second is programmatic, so it loads and ranks its tile while the first runs, and
-// waits for that one's end before it adds up.
+// Where few words are exchanged, always in this kernel, the rows come from
+// split_counts_kernel (arrived null): two plain launches, no memset and no waiting
+// among blocks.  The second is programmatic, so it loads and ranks its tile while the
+// first runs, and waits for that one's end before it adds up.  Otherwise
+// split_index_kernel is one cooperative launch: a tile's counts come from its own
+// ranking, are published as its row, and are added up once every block has arrived at
+// *fused.arrived (bounded wait).
 struct FusedArgs {
   unsigned *arrived;      // zeroed before the launch; null: his is the counts kernel's
   int32_t *his;           // [tiles][buckets]
@@ -768,28 +769,20 @@ int launch_scatter(const SplitArgs &a, int64_t tiles, int64_t stride, const int3
   return launch_status();
 }
 
-// The fused split with tiles of TILE elements; EDPP_ENOMEM (nothing launched)
-// when the tiles cannot all be resident or the cooperative launch is refused.
+// The fused split (position staging) with tiles of TILE elements; EDPP_ENOMEM
+// (nothing launched) when the tiles cannot all be resident or the cooperative launch
+// is refused.  Splits of fewer buckets never get here: while their tiles are all
+// resident they exchange fewer than kCountedWords words.
 template <int LAYOUT, int TILE>
 int launch_fused(const SplitArgs &a, char *ws, cudaStream_t st) {
-  constexpr auto index = split_index_kernel<LAYOUT, TILE, true>;
-  constexpr auto scatter = split_scatter_kernel<kScatterThreads, LAYOUT, TILE, true>;
-  const bool by_index = a.buckets >= index_buckets<LAYOUT>();
+  constexpr auto kernel = split_index_kernel<LAYOUT, TILE, true>;
+  if (a.buckets < index_buckets<LAYOUT>()) return EDPP_ENOMEM;
   int64_t resident = 0;
-  int s;
-  if (!by_index) {
-    s = prepare_kernel<scatter>(
-        kScatterThreads, scatter_smem_bytes<kScatterThreads, LAYOUT, TILE>(index_buckets<LAYOUT>(), true),
-        &resident);
-  } else if (a.buckets > 256) {
-    s = prepare_kernel<index>(kIndexThreads, index_smem_bytes<LAYOUT, TILE>(kOnePassMax),
-                                    &resident);
-  } else {
-    // the limit stays at the larger count's
-    s = prepare_kernel<index>(kIndexThreads, index_smem_bytes<LAYOUT, TILE>(kOnePassMax),
-                                    nullptr);
-    if (s == EDPP_OK) s = blocks_that_fit<index>(kIndexThreads, index_smem_bytes<LAYOUT, TILE>(256), &resident);
-  }
+  int s = prepare_kernel<kernel>(kIndexThreads, index_smem_bytes<LAYOUT, TILE>(kOnePassMax),
+                                 &resident);
+  // up to 256 buckets more of them fit; the limit stays at the larger count's
+  if (s == EDPP_OK && a.buckets <= 256)
+    s = blocks_that_fit<kernel>(kIndexThreads, index_smem_bytes<LAYOUT, TILE>(256), &resident);
   int64_t tiles = (a.n + TILE - 1) / TILE;
   if (s != EDPP_OK || tiles > resident) return EDPP_ENOMEM;
   if (cudaMemsetAsync(ws, 0, 16, st) != cudaSuccess) return EDPP_ECUDA;
@@ -797,19 +790,13 @@ int launch_fused(const SplitArgs &a, char *ws, cudaStream_t st) {
   const int32_t *his = nullptr;
   FusedArgs fused{reinterpret_cast<unsigned *>(ws), reinterpret_cast<int32_t *>(ws + 256),
                   a.bucket_start};
-  bool flag = by_index ? a.exact : bulk_runs<LAYOUT>(a);
   uint64_t timeout_ns = kDefaultWaitNs;
   unsigned *fault = fault_word();
   void *args[] = {&v.keys_in, &v.keys_out, &v.vals_in, &v.vals_out, &v.n,   &v.buckets, &v.shift,
-                  &tiles,     &his,        &v.tma,     &flag,       &timeout_ns, &fault, &fused};
-  const size_t smem = by_index
-                          ? index_smem_bytes<LAYOUT, TILE>(a.buckets)
-                          : scatter_smem_bytes<kScatterThreads, LAYOUT, TILE>(a.buckets, flag);
-  if (cudaLaunchCooperativeKernel(by_index ? reinterpret_cast<const void *>(index)
-                                           : reinterpret_cast<const void *>(scatter),
-                                  dim3(static_cast<unsigned>(tiles)),
-                                  dim3(by_index ? kIndexThreads : kScatterThreads), args, smem,
-                                  st) != cudaSuccess) {
+                  &tiles,     &his,        &v.tma,     &v.exact,    &timeout_ns, &fault, &fused};
+  if (cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(kernel),
+                                  dim3(static_cast<unsigned>(tiles)), dim3(kIndexThreads), args,
+                                  index_smem_bytes<LAYOUT, TILE>(a.buckets), st) != cudaSuccess) {
     cudaGetLastError();
     return EDPP_ENOMEM;
   }
