@@ -772,9 +772,11 @@ int launch_scatter(const SplitArgs &a, int64_t tiles, int64_t stride, const int3
 // The fused split (position staging) with tiles of TILE elements; EDPP_ENOMEM
 // (nothing launched) when the tiles cannot all be resident or the cooperative launch
 // is refused.  Splits of fewer buckets never get here: while their tiles are all
-// resident they exchange fewer than kCountedWords words.
+// resident they exchange fewer than kCountedWords words.  `missing` blocks are waited
+// for in vain (self-test).
 template <int LAYOUT, int TILE>
-int launch_fused(const SplitArgs &a, char *ws, cudaStream_t st) {
+int launch_fused(const SplitArgs &a, char *ws, cudaStream_t st,
+                 uint64_t timeout_ns = kDefaultWaitNs, int missing = 0) {
   constexpr auto kernel = split_index_kernel<LAYOUT, TILE, true>;
   if (a.buckets < index_buckets<LAYOUT>()) return EDPP_ENOMEM;
   int64_t resident = 0;
@@ -790,10 +792,10 @@ int launch_fused(const SplitArgs &a, char *ws, cudaStream_t st) {
   const int32_t *his = nullptr;
   FusedArgs fused{reinterpret_cast<unsigned *>(ws), reinterpret_cast<int32_t *>(ws + 256),
                   a.bucket_start};
-  uint64_t timeout_ns = kDefaultWaitNs;
   unsigned *fault = fault_word();
+  int64_t awaited = tiles + missing;
   void *args[] = {&v.keys_in, &v.keys_out, &v.vals_in, &v.vals_out, &v.n,   &v.buckets, &v.shift,
-                  &tiles,     &his,        &v.tma,     &v.exact,    &timeout_ns, &fault, &fused};
+                  &awaited,   &his,        &v.tma,     &v.exact,    &timeout_ns, &fault, &fused};
   if (cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(kernel),
                                   dim3(static_cast<unsigned>(tiles)), dim3(kIndexThreads), args,
                                   index_smem_bytes<LAYOUT, TILE>(a.buckets), st) != cudaSuccess) {
@@ -1108,6 +1110,23 @@ extern "C" int edpp_selftest_split_exact(const int32_t *keys_in, int32_t *keys_o
                                             : split_layout<EDPP_KVS_AOS>;
   return run(keys_in, keys_out, bucket_start, length, buckets, vals_in, vals_out, ws, ws_bytes,
              as_stream(stream), 0, /*exact=*/true);
+}
+
+// The fused split of keys, waiting for one block that is not there.
+extern "C" int edpp_selftest_split_timeout(const int32_t *keys_in, int32_t *keys_out, int64_t length,
+                                           int buckets, uint64_t timeout_ns, void *ws,
+                                           size_t ws_bytes, void *stream) {
+  using namespace edpp;
+  if (length <= 0 || length > INT32_MAX || !keys_in || !keys_out || timeout_ns == 0)
+    return EDPP_EINVAL;
+  if (buckets < index_buckets<EDPP_KO>() || buckets > kOnePassMax || (buckets & (buckets - 1)))
+    return EDPP_EINVAL;
+  if ((length + kSmallTile - 1) / kSmallTile * buckets > kFusedWords) return EDPP_EINVAL;
+  if (!ws || !aligned16(ws) || ws_bytes < split_ws_bytes(length, buckets)) return EDPP_ENOMEM;
+  const SplitArgs a{keys_in, keys_out, nullptr, nullptr, nullptr, length, buckets, 0,
+                    aligned16(keys_in), false};
+  return launch_fused<EDPP_KO, kSmallTile>(a, static_cast<char *>(ws), as_stream(stream),
+                                           timeout_ns, /*missing=*/1);
 }
 
 // ---- LSD radix sort on the stable split -----------------------------------------

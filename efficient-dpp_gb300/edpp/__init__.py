@@ -83,6 +83,7 @@ SIGNATURES = {
     "edpp_stream_triad_i32": (_I, [_VP, _VP, _VP, ctypes.c_int32, _I64, _VP]),
     "edpp_selftest_lookback_timeout": (_I, [_VP, _VP, _I64, _U64, _VP, _SZ, _VP]),
     "edpp_selftest_scan_pipe_timeout": (_I, [_VP, _VP, _I64, _U64, _VP, _SZ, _VP]),
+    "edpp_selftest_split_timeout": (_I, [_VP, _VP, _I64, _I, _U64, _VP, _SZ, _VP]),
     "edpp_selftest_split_exact": (_I, [_VP, _VP, _VP, _I64, _I, _I, _VP, _VP, _VP, _SZ, _VP]),
     "edpp_scan_exclusive_i32_noalloc": (_I, [_VP, _VP, _I64, _VP]),
     "edpp_scan_exclusive_i32_noalloc_max_length": (_I64, []),

@@ -564,6 +564,14 @@ int edpp_selftest_lookback_timeout(const int32_t *in, int32_t *out,
                                    int64_t length, uint64_t timeout_ns,
                                    void *ws, size_t ws_bytes, void *stream);
 
+/* The same for the one-launch split of keys (32 to 1024 buckets, at most 65536
+ * words: tiles of 2048 times buckets): every block waits for one more than there
+ * are, gives up, and no element is written.  ws of edpp_split_workspace_size,
+ * 16-byte aligned. */
+int edpp_selftest_split_timeout(const int32_t *keys_in, int32_t *keys_out,
+                                int64_t length, int buckets, uint64_t timeout_ns,
+                                void *ws, size_t ws_bytes, void *stream);
+
 /* The same for the pipelined one-launch scan (in and out 16-byte aligned): the
  * sum of the first tile is never published, so every block gives up and no
  * element is written.  ws of edpp_scan_workspace_size for the look-back scan. */
