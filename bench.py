@@ -88,10 +88,11 @@ def call_bytes(name, n):
 
 def call_launches(name, p, method="tiled"):
     """An upper bound on the kernels of this library one call launches, as the
-    step's accounting counts them; kernel_launches gives the kernels themselves."""
+    step's accounting counts them (the tiled gather as the seven of its former two-level
+    form); kernel_launches gives the kernels themselves."""
     if name not in ("gather", "scatter"):
         return 1
-    if method == "tiled":  # count, scan, partition, refine, (fetch, refine,) apply
+    if method == "tiled":  # scatter: count, scan, partition, refine, apply
         return 7 if name == "gather" else 5
     if method == "sweep" or p == 1:
         return p
@@ -801,8 +802,8 @@ def run_split_workload(args, rank, world):
 
 def run_autotune_workload(args, rank, world):
     """Per-size-class autotuning of the plain primitives: for every size
-    class, time each look-back tile shape and each slice length of the
-    chunked reduce-then-scan (int32 and int64), and the gather's tiled form
+    class, time the form of the length, each look-back tile shape and each slice
+    length of the chunked reduce-then-scan (int32 and int64), and the gather's tiled form
     against its direct sweep, on seeded data; record the winners and write
     the table (--tune-out, default the committed
     efficient-dpp_gb300/tuning/plain_gb300.tsv).  Prints every variant's time."""
