@@ -234,26 +234,28 @@ def _gs(kind, inp, loc, passes, out, method, ws):
         raise ValueError("inp shorter than loc")
     if out is None:
         out = torch.zeros(n, dtype=torch.int32, device=loc.device)
-    st = _stream()
-    src, dst, idx = _p(inp), _p(out), _p(loc)
+    st, L = _stream(), lib()
+    src, dst, idx = inp.data_ptr(), out.data_ptr(), loc.data_ptr()
     if method == "auto":  # the faster schedule for this size
+        method = "tiled"
         if kind == "gather":
-            direct = lib().edpp_gather_prefers_direct(n)
-        else:  # a sweep writes while it reads; the tiled scatter reads inp and loc first
-            direct = (abs(src - dst) >= 4 * n and abs(idx - dst) >= 4 * n
-                      and lib().edpp_scatter_prefers_direct(n))
-        method = "sweep" if direct else "tiled"
-        passes = 1 if method == "sweep" else passes
+            if L.edpp_gather_prefers_direct(n):
+                method, passes = "sweep", 1
+        elif L.edpp_scatter_prefers_direct(n):
+            # a sweep writes while it reads; the tiled scatter reads inp and loc first
+            a, b, size = dst - src, dst - idx, 4 * n
+            if (a >= size or -a >= size) and (b >= size or -b >= size):
+                method, passes = "sweep", 1
     if method == "sweep":
-        f = lib().edpp_gather_i32 if kind == "gather" else lib().edpp_scatter_i32
+        f = L.edpp_gather_i32 if kind == "gather" else L.edpp_scatter_i32
         check(f(src, dst, n, idx, int(passes), st), kind)
     elif method in ("partition", "tiled"):
         if ws is None:
             ws = workspace(gs_workspace_bytes(kind, n, passes, method), loc.device)
         if method == "partition":
-            f = lib().edpp_gather_i32_ws if kind == "gather" else lib().edpp_scatter_i32_ws
+            f = L.edpp_gather_i32_ws if kind == "gather" else L.edpp_scatter_i32_ws
         else:
-            f = lib().edpp_gather_i32_tiled if kind == "gather" else lib().edpp_scatter_i32_tiled
+            f = L.edpp_gather_i32_tiled if kind == "gather" else L.edpp_scatter_i32_tiled
         check(f(src, dst, n, idx, int(passes), _p(ws), ws.numel(), st), kind)
     else:
         raise ValueError(method)
